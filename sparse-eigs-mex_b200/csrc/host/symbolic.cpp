@@ -642,68 +642,109 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
             fs_par[s] = (par[last] == -1) ? -1 : fs_of[par[last]];
         }
 
-        // ---- 7. relaxed amalgamation (bottom-up; merge a child into its
-        // parent when the child's columns immediately precede the parent's)
-        std::vector<int32_t> mfirst(fs_first.begin(), fs_first.end() - 1);  // current first col
-        std::vector<int32_t> mcols(nfs), mrows(nfs), rep(nfs);
+        // ---- 7. relaxed amalgamation: bottom-up, any child may be merged into
+        // its parent (not only the one whose columns happen to precede the
+        // parent's), and the columns are then renumbered so that every merged
+        // supernode is a contiguous range.  The renumbering is a topological
+        // order of the same elimination tree, so the factor's structure does
+        // not change, only the explicit zeros that the merges admit.
+        std::vector<int32_t> mcols(nfs), mrows(nfs), grp(nfs);
         std::vector<double> mzeros(nfs, 0.0);
         for (int32_t s = 0; s < nfs; s++) {
             mcols[s] = fs_first[s + 1] - fs_first[s];
             mrows[s] = (int32_t)cc[fs_first[s]];
-            rep[s] = s;
+            grp[s] = s;
         }
-        // rep[s]: the fundamental supernode that now heads s's merged group
-        // (groups are merged upward; the parent's record stays the live one)
-        std::vector<char> absorbed(nfs, 0);
         for (int32_t s = 0; s < nfs; s++) {
-            int32_t p = fs_par[s];
+            const int32_t p = fs_par[s];
             if (p < 0) continue;
-            // live group of p is p itself (p has not been absorbed yet, since
-            // p > s in postorder and merging only goes upward)
-            int32_t cs = mcols[s], cp = mcols[p];
-            if (mfirst[s] + cs != mfirst[p]) continue;  // not contiguous
-            int32_t rs = mrows[s], rp = mrows[p];
-            int32_t ns = cs + cp;
-            int32_t rnew = cs + rp;
-            double newz = (double)cs * (double)(cs + rp - rs);
-            double totz = mzeros[s] + mzeros[p] + newz;
-            double denom = (double)ns * (ns + 1) / 2.0 + (double)ns * (double)(rnew - ns);
-            double z = denom > 0 ? totz / denom : 0.0;
-            bool merge = (ns <= 4) || (ns <= 16 && z < 0.8) || (ns <= 48 && z < 0.1) ||
-                         (z < 0.05);
+            // p has not been merged yet (p > s in postorder, and merging only
+            // goes upward), so it is the live record of its group
+            const int32_t cs = mcols[s], ns = cs + mcols[p], rnew = cs + mrows[p];
+            const double newz = (double)cs * (double)(rnew - mrows[s]);
+            const double totz = mzeros[s] + mzeros[p] + newz;
+            const double denom = (double)ns * (ns + 1) / 2.0 + (double)ns * (double)(rnew - ns);
+            const double z = denom > 0 ? totz / denom : 0.0;
+            // The narrower the merged supernode, the larger the share of zeros
+            // it may hold: a tree level costs the solves and the factor a
+            // fixed hand-over, extra entries only bandwidth.  48^3 grid: 47,615
+            // supernodes in 21 levels when only a child whose columns precede
+            // its parent's could merge, 3,053 in 15 levels now, 24 % more
+            // entries; 30 block solves of 8 columns 16.0 -> 13.3 ms (narrower
+            // limits 32/64/64: 14.2, 24/48/64: 15.2).
+            const bool merge = (ns <= 48 && z < 0.8) || (ns <= 96 && z < 0.4) ||
+                               (ns <= 128 && z < 0.2) || z < 0.05;
             if (!merge) continue;
-            mfirst[p] = mfirst[s];
             mcols[p] = ns;
             mrows[p] = rnew;
             mzeros[p] = totz;
-            absorbed[s] = 1;
+            grp[s] = p;
         }
-        // final supernodes: the non-absorbed fundamental ones, in column order
-        std::vector<int32_t> fin_of_fs(nfs, -1);
-        std::vector<int32_t> sf;
-        for (int32_t s = 0; s < nfs; s++) {
-            if (absorbed[s]) continue;
-            fin_of_fs[s] = (int32_t)sf.size();
-            sf.push_back(mfirst[s]);
+        for (int32_t s = nfs - 1; s >= 0; s--)
+            if (grp[s] != s) grp[s] = grp[grp[s]];   // the parent's group is final
+        // groups in postorder of the merged tree: a group follows every group
+        // below it, and its columns keep their order among themselves
+        std::vector<int32_t> gpar(nfs, -1), ghead(nfs, -1), gnext(nfs, -1), glast(nfs, -1);
+        std::vector<int32_t> mhead(nfs, -1), mnext(nfs, -1);
+        for (int32_t s = nfs - 1; s >= 0; s--) {
+            mnext[s] = mhead[grp[s]];
+            mhead[grp[s]] = s;
+            if (grp[s] != s) continue;
+            gpar[s] = fs_par[s] < 0 ? -1 : grp[fs_par[s]];
+            if (gpar[s] >= 0) {
+                gnext[s] = ghead[gpar[s]];
+                ghead[gpar[s]] = s;
+            }
         }
-        const int32_t ns = (int32_t)sf.size();
-        // sort by first column (postorder guarantees increasing already, but be safe)
-        std::vector<int32_t> order(ns);
-        for (int32_t i = 0; i < ns; i++) order[i] = i;
-        std::sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return sf[a] < sf[b]; });
-        std::vector<int32_t> rank(ns);
-        for (int32_t i = 0; i < ns; i++) rank[order[i]] = i;
+        std::vector<int32_t> gorder;                 // groups, children first
+        gorder.reserve(nfs);
+        {
+            std::vector<int32_t> stk;
+            for (int32_t r = 0; r < nfs; r++) {
+                if (grp[r] != r || gpar[r] >= 0) continue;
+                stk.push_back(r);
+                while (!stk.empty()) {
+                    const int32_t g = stk.back(), c = ghead[g];
+                    if (c < 0) {
+                        gorder.push_back(g);
+                        stk.pop_back();
+                    } else {
+                        ghead[g] = gnext[c];
+                        stk.push_back(c);
+                    }
+                }
+            }
+        }
+        const int32_t ns = (int32_t)gorder.size();
         S->nsuper = ns;
         S->sfirst = xalloc<int32_t>(ns + 1);
-        for (int32_t i = 0; i < ns; i++) S->sfirst[i] = sf[order[i]];
-        S->sfirst[ns] = n;
         S->col2sup = xalloc<int32_t>(n);
-        for (int32_t s = 0; s < ns; s++)
-            for (int32_t j = S->sfirst[s]; j < S->sfirst[s + 1]; j++) S->col2sup[j] = s;
         S->sparent = xalloc<int32_t>(ns);
-        for (int32_t s = 0; s < ns; s++) {
-            int32_t last = S->sfirst[s + 1] - 1;
-            S->sparent[s] = (par[last] == -1) ? -1 : S->col2sup[par[last]];
+        std::vector<int32_t> rank(nfs, -1), oldcol(n), newcol(n);
+        {
+            int32_t k = 0;
+            for (int32_t i = 0; i < ns; i++) {
+                rank[gorder[i]] = i;
+                S->sfirst[i] = k;
+                for (int32_t f = mhead[gorder[i]]; f >= 0; f = mnext[f])
+                    for (int32_t j = fs_first[f]; j < fs_first[f + 1]; j++, k++) {
+                        oldcol[k] = j;
+                        newcol[j] = k;
+                        S->col2sup[k] = i;
+                    }
+            }
+            S->sfirst[ns] = n;
+            for (int32_t i = 0; i < ns; i++)
+                S->sparent[i] = gpar[gorder[i]] < 0 ? -1 : rank[gpar[gorder[i]]];
+        }
+        {
+            std::vector<int32_t> op(S->perm, S->perm + n);
+            spx::parallel_ranges(n, kGrain, [&](int64_t lo, int64_t hi) {
+                for (int64_t k = lo; k < hi; k++) {
+                    S->perm[k] = op[oldcol[k]];
+                    S->iperm[S->perm[k]] = (int32_t)k;
+                }
+            });
         }
 
         // ---- 8. row structure of every supernode
@@ -728,8 +769,7 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
         // come out at another length, every list is built again into
         // separate vectors and the offsets follow the lists.
         std::vector<int64_t> rptr(ns + 1, 0);
-        for (int32_t s = 0; s < nfs; s++)
-            if (!absorbed[s]) rptr[rank[fin_of_fs[s]] + 1] = mrows[s];
+        for (int32_t i = 0; i < ns; i++) rptr[i + 1] = mrows[gorder[i]];
         for (int32_t s = 0; s < ns; s++) rptr[s + 1] += rptr[s];
         S->rows = xalloc<int32_t>(rptr[ns]);
         std::vector<std::vector<int32_t>> rs;          // only when a prediction fails
@@ -739,8 +779,9 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
             int32_t f = S->sfirst[s], l = S->sfirst[s + 1];
             tmp.clear();
             for (int32_t j = f; j < l; j++) {
-                for (int64_t p = prp[j]; p < prp[j + 1]; p++) {
-                    int32_t i = pci[p];
+                const int32_t oj = oldcol[j];
+                for (int64_t p = prp[oj]; p < prp[oj + 1]; p++) {
+                    int32_t i = newcol[pci[p]];
                     if (i >= l && mark[i] != s) { mark[i] = s; tmp.push_back(i); }
                 }
             }
@@ -777,7 +818,7 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
                 if (p >= 0 && fdesc[s] < fdesc[p]) fdesc[p] = fdesc[s];
             }
             const unsigned hw = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
-            const int32_t target = std::max<int32_t>(256, ns / (int32_t)(4 * hw));
+            const int32_t target = std::max<int32_t>(16, ns / (int32_t)(4 * hw));
             std::vector<char> in_task(ns, 0);
             std::vector<int32_t> task_root;
             std::vector<int32_t> stack;
@@ -794,7 +835,7 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
             }
             for (int32_t r : task_root)
                 for (int32_t s = fdesc[r]; s <= r; s++) in_task[s] = 1;
-            const unsigned nth = (hw > 1 && ns > 2048) ? hw : 1u;
+            const unsigned nth = (hw > 1 && n > 16384) ? hw : 1u;
             auto build_all = [&] {
                 std::atomic<size_t> next{0};
                 auto worker = [&] {
@@ -835,7 +876,7 @@ extern "C" int spx_analyze(int32_t n, const int64_t *rowptr, const int32_t *col,
         // (every child has one parent, so the parents' writes are disjoint)
         S->relmap = xalloc<int32_t>(nrows_total);
         std::fill(S->relmap, S->relmap + nrows_total, -1);
-        spx::parallel_ranges(ns, kGrain, [&](int64_t lo, int64_t hi) {
+        spx::parallel_ranges(ns, 128, [&](int64_t lo, int64_t hi) {
             std::vector<int32_t> pos(n, -1);
             for (int64_t p = lo; p < hi; p++) {
                 if (cptr[p] == cptr[p + 1]) continue;

@@ -1,22 +1,10 @@
 // Device multifrontal supernodal Cholesky (FP64) and the task-queue
 // shift-invert solve.  See multifrontal.cuh for the storage scheme.
 //
-// Factorization of one tree level.  Fronts of at most 32 rows are done by
-// one warp each (mf_tiny_front).  Larger fronts are assembled on 32 x 32
-// tiles and factored on 64 x 64 tiles (pivot tiles first, then the tiles of
-// the rows below the pivots), every tile product on the FP64 tensor cores:
-//   assemble  F = A(pivot columns) + shift*I + extend-add of the children's
-//             update matrices (pulled per tile, children in a fixed order)
-//   for kb:   diag: Cholesky + inverse of the diagonal tile kb (inv into
-//             G); rows: the tiles below it as L_Ik = F_Ik inv(L_kk)^T;
-//             update of column block kb+1, then of the other trailing
-//             tiles, update matrix included.  diag and rows run on a
-//             high-priority second branch of the factor graph, so the
-//             diagonal step kb+1 overlaps the rest of update kb.
-//   invert    the off-diagonal tiles of inv(L11) by recursive doubling
-//   wmul      G's lower part = L21 * inv(L11)
-// A pivot that is not positive records the failing column in a device status
-// word (never a trap); later kernels of the same factorization return early.
+// The factorization is one persistent kernel over 64 x 64 tile tasks
+// (mf_factor.cuh); the solve pair is another over panel tiles (below).  A
+// pivot that is not positive records the failing column in a device status
+// word (never a trap); the tasks after it do no work.
 #include "multifrontal.cuh"
 #include "../common.cuh"
 #include "../counters.h"
@@ -50,895 +38,6 @@ constexpr int kLdgA = (int)(16 / sizeof(Real));
 cudaMemPool_t device_pool(int dev);
 
 namespace {
-
-constexpr int T = kTile;
-constexpr int kFThreads = 256;
-
-struct Sym {
-    const int32_t *sfirst, *rows, *relmap, *child_ptr, *child_list;
-    const int64_t *rowptr, *frontptr, *gptr;
-    // per child: for each 32-row tile boundary of its parent, the first
-    // entry of the child's update rows that maps at or below it
-    const int32_t *cbnd;
-    const int64_t *cbnd_ptr;
-};
-
-struct Front {
-    int64_t fptr, gptr;
-    int r, c, nkb, nt, first;
-    int ldg;          // leading dimension of the G panel: r rounded up to 16 bytes
-};
-
-// Front geometry with tiles of TS rows/columns: pivot tiles first, then the
-// tiles of the rows below the pivots.
-template <int TS>
-SPX_DEV Front front_of(const Sym &y, int s) {
-    Front f;
-    f.first = y.sfirst[s];
-    f.c = y.sfirst[s + 1] - f.first;
-    f.r = (int)(y.rowptr[s + 1] - y.rowptr[s]);
-    f.nkb = (f.c + TS - 1) / TS;
-    f.nt = f.nkb + (f.r - f.c + TS - 1) / TS;
-    f.fptr = y.frontptr[s];
-    f.gptr = y.gptr[s];
-    f.ldg = (f.r + kLdgA - 1) & ~(kLdgA - 1);
-    return f;
-}
-
-template <int TS>
-SPX_DEV void tile_range(const Front &f, int I, int &a, int &b) {
-    if (I < f.nkb) { a = I * TS; b = min(a + TS, f.c); }
-    else { a = f.c + (I - f.nkb) * TS; b = min(a + TS, f.r); }
-}
-
-// ------------------------------------------------------------ assemble --
-__global__ void __launch_bounds__(kFThreads)
-mf_assemble(const int4 *__restrict__ tasks, Sym y, Real *__restrict__ F,
-            const int32_t *__restrict__ acolptr, const int32_t *__restrict__ atpos,
-            const int32_t *__restrict__ asrc, const double *__restrict__ val,
-            const double *__restrict__ params, const int *status) {
-    __shared__ double S[T][T + 1];
-    if (*(volatile const int *)status) return;
-    const double shift = params[0];
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, I = tk.y, J = tk.z;
-    const Front f = front_of<T>(y, s);
-    int ra, rb, ca, cb;
-    tile_range<T>(f, I, ra, rb);
-    tile_range<T>(f, J, ca, cb);
-    const int h = rb - ra, w = cb - ca;
-    // The children's geometry is read by one thread per child, a batch of
-    // kFThreads children at a time, and the children that touch this tile
-    // are listed in child order; only those are added, one after another
-    // (a parent entry can receive several children's terms, and the fixed
-    // order keeps the sums reproducible).
-    __shared__ int s_ch[kFThreads], s_ia[kFThreads], s_ja[kFThreads], s_hw[kFThreads];
-    __shared__ int s_cnt;
-    for (int t = threadIdx.x; t < T * T; t += blockDim.x) S[t & (T - 1)][t >> 5] = 0.0;
-    const int q0 = y.child_ptr[s], q1 = y.child_ptr[s + 1];
-    for (int qb = q0; qb < q1; qb += kFThreads) {
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-        const int q = qb + (int)threadIdx.x;
-        int ch = -1, ia = 0, ja = 0, hi = 0, wj = 0;
-        if (q < q1) {
-            ch = y.child_list[q];
-            const int32_t *bd = y.cbnd + y.cbnd_ptr[ch];
-            ia = bd[I];
-            hi = bd[I + 1] - ia;
-            ja = bd[J];
-            wj = bd[J + 1] - ja;
-        }
-        const bool live = hi > 0 && wj > 0;
-        // order-preserving compaction: warp ballots, then the warps' counts
-        const unsigned bal = __ballot_sync(0xffffffffu, live);
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        __shared__ int s_wcnt[kFThreads / 32];
-        if (lane == 0) s_wcnt[wid] = __popc(bal);
-        __syncthreads();
-        if (live) {
-            int pos = __popc(bal & ((1u << lane) - 1u));
-            for (int w2 = 0; w2 < wid; w2++) pos += s_wcnt[w2];
-            s_ch[pos] = ch;
-            s_ia[pos] = ia;
-            s_ja[pos] = ja;
-            s_hw[pos] = hi | (wj << 16);
-        }
-        if (threadIdx.x == 0) {
-            int tot = 0;
-            for (int w2 = 0; w2 < kFThreads / 32; w2++) tot += s_wcnt[w2];
-            s_cnt = tot;
-        }
-        __syncthreads();
-        const int cnt = s_cnt;
-        for (int e = 0; e < cnt; e++) {
-            const int c2 = s_ch[e], ia2 = s_ia[e], ja2 = s_ja[e];
-            const int hi2 = s_hw[e] & 0xffff, wj2 = s_hw[e] >> 16;
-            const int rch = (int)(y.rowptr[c2 + 1] - y.rowptr[c2]);
-            const int cch = y.sfirst[c2 + 1] - y.sfirst[c2];
-            const int32_t *rm = y.relmap + y.rowptr[c2] + cch;
-            const Real *U = F + y.frontptr[c2];
-            for (int t = threadIdx.x; t < hi2 * wj2; t += blockDim.x) {
-                const int i = ia2 + t % hi2, j = ja2 + t / hi2;
-                if (i >= j)
-                    S[rm[i] - ra][rm[j] - ca] += U[(int64_t)(cch + i) + (int64_t)(cch + j) * rch];
-            }
-            __syncthreads();
-        }
-    }
-    __syncthreads();
-    if (J < f.nkb) {
-        if (threadIdx.x < w) {
-            const int jj = ca + threadIdx.x;
-            const int col = f.first + jj;
-            for (int e = acolptr[col]; e < acolptr[col + 1]; e++) {
-                const int tp = atpos[e];
-                if (tp >= ra && tp < rb) S[tp - ra][threadIdx.x] += val[asrc[e]];
-            }
-            if (I == J) S[jj - ra][threadIdx.x] += shift;
-        }
-    }
-    __syncthreads();
-    Real *Fs = F + f.fptr;
-    for (int t = threadIdx.x; t < T * T; t += blockDim.x) {
-        const int i = t & (T - 1), j = t >> 5;
-        if (i < h && j < w) Fs[(int64_t)(ra + i) + (int64_t)(ca + j) * f.r] = (Real)S[i][j];
-    }
-}
-
-// ------------------------------------------------------ warp Cholesky --
-// Shared by the diagonal-tile POTRF and the tiny-front kernel: one warp,
-// lane i owns row i of M (n <= 32 rows in shared memory).  The scaled column
-// j is published in its own array `col`, so the rank-1 updates read it
-// without aliasing the rows being updated.  Factors the first c columns of
-// the n x n lower matrix M in place (rows >= c receive L21 and the Schur
-// complement) and sets dinv[j] = 1 / L(j, j); a pivot <= pivtol records its
-// column in *status and is replaced by 1 so the sweep stays finite.
-SPX_DEV void warp_cholesky(double (*M)[T + 1], double *col, double *dinv, int n, int c,
-                           double pivtol, int *status, int colbase) {
-    const int lane = threadIdx.x & 31;
-    for (int j = 0; j < c; j++) {
-        if (lane == j) {
-            double d = M[j][j];
-            if (!(d > pivtol)) {
-                atomicCAS(status, 0, colbase + j + 1);
-                d = 1.0;
-            }
-            d = sqrt(d);
-            M[j][j] = d;
-            dinv[j] = 1.0 / d;
-        }
-        __syncwarp();
-        double lij = 0.0;
-        if (lane > j && lane < n) {
-            lij = M[lane][j] * dinv[j];
-            M[lane][j] = lij;
-            col[lane] = lij;
-        }
-        __syncwarp();
-        if (lane > j && lane < n)
-            for (int k = j + 1; k <= lane; k++) M[lane][k] -= lij * col[k];
-        __syncwarp();
-    }
-}
-
-// X = inv(L11) for the leading c x c block of M, kept in M's strictly upper
-// part: X(i, j) for i > j sits at M[j][i] (lane j computes column j), and
-// X(j, j) = dinv[j].  The lower part (L) is left as it is.
-SPX_DEV void warp_tri_inverse(double (*M)[T + 1], const double *dinv, int c) {
-    const int j = threadIdx.x & 31;
-    if (j < c) {
-        for (int i = j + 1; i < c; i++) {
-            double acc = M[i][j] * dinv[j];
-            for (int t2 = j + 1; t2 < i; t2++) acc += M[i][t2] * M[j][t2];
-            M[j][i] = -acc * dinv[i];
-        }
-    }
-    __syncwarp();
-}
-
-// ---------------------------------------------------------- tiny front --
-// A front with at most 32 rows is done by one warp end to end: assembly
-// (children's update matrices, then A and the shift), partial Cholesky of its
-// c pivots with the Schur complement left in the rows below, the update
-// matrix written back for the parent, then X = inv(L11) and W = L21 X into G.
-constexpr int kTinyWarps = 4;
-
-__global__ void __launch_bounds__(32 * kTinyWarps)
-mf_tiny_front(const int4 *__restrict__ tasks, int ntasks, Sym y, Real *__restrict__ F,
-              Real *__restrict__ G, const int32_t *__restrict__ acolptr,
-              const int32_t *__restrict__ atpos, const int32_t *__restrict__ asrc,
-              const double *__restrict__ val, const double *__restrict__ params, int *status) {
-    __shared__ double Ms[kTinyWarps][T][T + 1];
-    __shared__ double cols[kTinyWarps][T], dinvs[kTinyWarps][T];
-    if (*(volatile int *)status) return;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int task = blockIdx.x * kTinyWarps + wid;
-    if (task >= ntasks) return;
-    const double shift = params[0];
-    const int s = tasks[task].x;
-    const Front f = front_of<T>(y, s);
-    const int r = f.r, c = f.c;
-    double (*M)[T + 1] = Ms[wid];
-    for (int k = 0; k < T; k++) M[lane][k] = 0.0;
-    __syncwarp();
-    for (int q = y.child_ptr[s]; q < y.child_ptr[s + 1]; q++) {
-        const int ch = y.child_list[q];
-        const int rch = (int)(y.rowptr[ch + 1] - y.rowptr[ch]);
-        const int cch = y.sfirst[ch + 1] - y.sfirst[ch];
-        const int nb = rch - cch;
-        const int32_t *rm = y.relmap + y.rowptr[ch] + cch;
-        const Real *U = F + y.frontptr[ch];
-        for (int e = lane; e < nb * nb; e += 32) {
-            const int a2 = e % nb, b2 = e / nb;
-            if (a2 >= b2) M[rm[a2]][rm[b2]] += U[(int64_t)(cch + a2) + (int64_t)(cch + b2) * rch];
-        }
-        __syncwarp();
-    }
-    if (lane < c) {
-        const int col = f.first + lane;
-        for (int e = acolptr[col]; e < acolptr[col + 1]; e++) M[atpos[e]][lane] += val[asrc[e]];
-        M[lane][lane] += shift;
-    }
-    __syncwarp();
-    warp_cholesky(M, cols[wid], dinvs[wid], r, c, params[1], status, f.first);
-    // update matrix (rows and columns c..r-1) for the parent's assembly
-    Real *Fs = F + f.fptr;
-    if (lane >= c && lane < r)
-        for (int k = c; k <= lane; k++) Fs[(int64_t)lane + (int64_t)k * r] = (Real)M[lane][k];
-    const double *dinv = dinvs[wid];
-    warp_tri_inverse(M, dinv, c);
-    Real *Gs = G + f.gptr;
-    if (lane < c) {
-        Gs[(int64_t)lane + (int64_t)lane * f.ldg] = (Real)dinv[lane];
-        for (int i = lane + 1; i < c; i++) Gs[(int64_t)i + (int64_t)lane * f.ldg] = (Real)M[lane][i];
-    }
-    // W = L21 X: lane i >= c owns row i
-    if (lane >= c && lane < r) {
-        for (int j = 0; j < c; j++) {
-            double acc = M[lane][j] * dinv[j];
-            for (int t2 = j + 1; t2 < c; t2++) acc += M[lane][t2] * M[j][t2];
-            Gs[(int64_t)lane + (int64_t)j * f.ldg] = (Real)acc;
-        }
-    }
-}
-
-// ------------------------------------------------------- factor tiles --
-// Fronts with more than 32 rows are factored on 64 x 64 tiles.  Every tile
-// product runs on the FP64 tensor cores (mma.sync m8n8k4 f64): a CTA of four
-// warps owns one 64 x 64 output tile, each warp a 32 x 32 quarter held as
-// 4 x 4 accumulator fragments.  Operand tiles are staged in shared memory
-// column-major with a leading dimension of 68 doubles, which makes both the
-// fragment reads (8 rows x 4 columns per warp) and the coalesced column
-// loads free of bank conflicts.
-constexpr int FT = 64;
-constexpr int FLD = 68;
-constexpr int kGThreads = 128;
-constexpr int kFTileDoubles = FT * FLD;
-constexpr int kPanelGroup = 4;   // panel tiles of a small front share one block
-constexpr size_t kPanelSmem = 4 * sizeof(double) * kFTileDoubles;   // mf_diag64
-constexpr size_t kRowsSmem = 3 * sizeof(double) * kFTileDoubles;    // mf_rows64
-constexpr size_t kPairSmem = 2 * sizeof(double) * kFTileDoubles;
-
-SPX_DEV void dmma(double &d0, double &d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
-}
-
-// Tile loads go through cp.async (one element per copy, zero-filled outside
-// the h x w block), so all of a thread's 32 element copies are in flight at
-// once; cp_wait() completes them and makes them visible to the block.
-SPX_DEV void cp_async8(double *dst, const double *src, bool valid) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(saddr), "l"(src),
-                 "r"(valid ? 8 : 0) : "memory");
-}
-SPX_DEV void cp_wait() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-}
-SPX_DEV void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// wait until at most one committed group (the most recent) is still in flight
-SPX_DEV void cp_wait_all_but_last() {
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-}
-SPX_DEV void cp_async4(float *dst, const float *src, bool valid) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(saddr), "l"(src),
-                 "r"(valid ? 4 : 0) : "memory");
-}
-// FP32 storage: element (i, j) of a tile is copied asynchronously (4 bytes)
-// to a 64 x 65 float staging area at the top of the tile's own storage,
-// float offset kStageOff + j * FST + i, and the tile is widened in place
-// once the copies are complete (tile_widen).  The staging area starts above
-// the FP64 columns 0 .. 31, so only the second half of the widening has to
-// wait until every staged float has been read.
-constexpr int FST = 65;
-constexpr int kStageOff = 2 * kFTileDoubles - FT * FST;
-static_assert(kStageOff * 4 >= 32 * FLD * 8, "staging area overlaps the first 32 columns");
-
-// one element of a tile (zero when !valid)
-template <class MT>
-SPX_DEV void elem_copy(double *s, int i, int j, const MT *src, bool valid) {
-    if constexpr (std::is_same<MT, double>::value) cp_async8(s + j * FLD + i, src, valid);
-    else cp_async4(reinterpret_cast<float *>(s) + kStageOff + j * FST + i, src, valid);
-}
-
-// Widen a staged FP32 tile to FP64 in place (a no-op for FP64 storage).  The
-// block's copies must be complete and visible (cp_wait); the caller
-// synchronises the block again before the tile is read.
-template <class MT>
-SPX_DEV void tile_widen(double *s) {
-    if constexpr (!std::is_same<MT, double>::value) {
-        constexpr int kPer = FT * FT / kGThreads, kHalf = kPer / 2;
-        const float *f = reinterpret_cast<const float *>(s) + kStageOff;
-        float hi[kHalf];
-#pragma unroll
-        for (int q = 0; q < kHalf; q++) {
-            const int t = threadIdx.x + (q + kHalf) * kGThreads;
-            hi[q] = f[(t >> 6) * FST + (t & (FT - 1))];
-        }
-#pragma unroll
-        for (int q = 0; q < kHalf; q++) {
-            const int t = threadIdx.x + q * kGThreads;
-            s[(t >> 6) * FLD + (t & (FT - 1))] = (double)f[(t >> 6) * FST + (t & (FT - 1))];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < kHalf; q++) {
-            const int t = threadIdx.x + (q + kHalf) * kGThreads;
-            s[(t >> 6) * FLD + (t & (FT - 1))] = (double)hi[q];
-        }
-    }
-}
-
-// complete the block's tile copies and make the tiles a (and b) readable
-template <class MT>
-SPX_DEV void tiles_ready(double *a, double *b = nullptr) {
-    cp_wait();
-    if constexpr (!std::is_same<MT, double>::value) {
-        tile_widen<MT>(a);
-        if (b) tile_widen<MT>(b);
-        __syncthreads();
-    }
-}
-
-// s(i, j) = M(ra + i, ca + j) for i < h, j < w; zero elsewhere in the tile
-template <class MT>
-SPX_DEV void ftile_load(double *s, const MT *M, int64_t ld, int ra, int h, int ca, int w) {
-#pragma unroll 8
-    for (int q = 0; q < FT * FT / kGThreads; q++) {
-        const int t = threadIdx.x + q * kGThreads;
-        const int i = t & (FT - 1), j = t >> 6;
-        const bool v = (i < h && j < w);
-        elem_copy(s, i, j, v ? M + (int64_t)(ra + i) + (int64_t)(ca + j) * ld : M, v);
-    }
-}
-// s(i, j) = M(ca + j, ra + i): the transpose of the stored block
-template <class MT>
-SPX_DEV void ftile_load_t(double *s, const MT *M, int64_t ld, int ra, int h, int ca, int w) {
-#pragma unroll 8
-    for (int q = 0; q < FT * FT / kGThreads; q++) {
-        const int t = threadIdx.x + q * kGThreads;
-        const int j = t & (FT - 1), i = t >> 6;
-        const bool v = (i < h && j < w);
-        elem_copy(s, i, j, v ? M + (int64_t)(ca + j) + (int64_t)(ra + i) * ld : M, v);
-    }
-}
-// lower triangle of the w x w block at (a, a); zero elsewhere
-template <class MT>
-SPX_DEV void ftile_load_lower(double *s, const MT *M, int64_t ld, int a, int w) {
-#pragma unroll 8
-    for (int q = 0; q < FT * FT / kGThreads; q++) {
-        const int t = threadIdx.x + q * kGThreads;
-        const int i = t & (FT - 1), j = t >> 6;
-        const bool v = (i < w && j <= i);
-        elem_copy(s, i, j, v ? M + (int64_t)(a + i) + (int64_t)(a + j) * ld : M, v);
-    }
-}
-
-using Acc = double[4][4][2];
-
-SPX_DEV void acc_zero(Acc &acc) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
-}
-
-// acc += A B^T (BT) or A B, with A a 64 x kw tile (s(i, k) at k*FLD + i) and
-// B given as 64 x kw (BT: B(n, k) at k*FLD + n) or kw x 64 (B(k, n) at n*FLD + k).
-// Only the fragments that touch the first mh rows / nw columns of the
-// output are computed (the rest of the accumulator stays zero).
-template <bool BT>
-SPX_DEV void warp_mma(Acc &acc, const double *As, const double *Bs, int kw, int mh = FT,
-                      int nw = FT) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int wid = threadIdx.x >> 5, m0 = (wid & 1) * 32, n0 = (wid >> 1) * 32;
-    if (m0 >= mh || n0 >= nw) return;
-    const int mi = min(4, (mh - m0 + 7) >> 3), nj = min(4, (nw - n0 + 7) >> 3);
-    for (int k = 0; k < kw; k += 4) {
-        double a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) a[i] = As[(k + t) * FLD + m0 + 8 * i + g];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            b[j] = BT ? Bs[(k + t) * FLD + n0 + 8 * j + g] : Bs[(n0 + 8 * j + g) * FLD + k + t];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (i < mi && j < nj) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-    }
-}
-
-// M(ra + m, ca + n) = alpha * acc(m, n) (+ M when add), for m < h, n < w.
-// TRANS stores acc(m, n) at M(ca + n, ra + m) instead.
-template <bool TRANS, class MT>
-SPX_DEV void acc_store(const Acc &acc, MT *M, int64_t ld, int ra, int h, int ca, int w,
-                       double alpha, bool add) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int wid = threadIdx.x >> 5, m0 = (wid & 1) * 32, n0 = (wid >> 1) * 32;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int m = m0 + 8 * i + g, n = n0 + 8 * j + 2 * t + e;
-                if (m < h && n < w) {
-                    MT *p = TRANS ? M + (int64_t)(ca + n) + (int64_t)(ra + m) * ld
-                                  : M + (int64_t)(ra + m) + (int64_t)(ca + n) * ld;
-                    *p = (MT)(add ? (double)*p + alpha * acc[i][j][e] : alpha * acc[i][j][e]);
-                }
-            }
-}
-
-// M(ra + m, ca + n) = Cs(m, n) - acc(m, n) for m < h, n < w (Cs: the staged
-// output tile, column-major FLD)
-template <class MT>
-SPX_DEV void acc_sub_store(const Acc &acc, const double *Cs, MT *M, int64_t ld, int ra, int h,
-                           int ca, int w) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int wid = threadIdx.x >> 5, m0 = (wid & 1) * 32, n0 = (wid >> 1) * 32;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int m = m0 + 8 * i + g, n = n0 + 8 * j + 2 * t + e;
-                if (m < h && n < w)
-                    M[(int64_t)(ra + m) + (int64_t)(ca + n) * ld] = (MT)(Cs[n * FLD + m] - acc[i][j][e]);
-            }
-}
-
-// ---- recursive Cholesky + inverse of a diagonal tile (w <= 64) --------
-// chol_inv_rec<N>: L (lower) and X = inv(L) of the leading w x w part of the
-// N x N lower matrix D (all column-major, leading dimension FLD), by the 128
-// threads of the block, 2 x 2 blocked down to 8 x 8:
-//   L00, X00 (recursive); L10 = A10 X00^T; A11 -= L10 L10^T and
-//   T = L10 X00 (one phase); L11, X11 (recursive); X10 = -X11 T.
-// The sequential chain is one 8 x 8 base case per 8 pivots; everything else
-// is small products spread over the block.  Rows/columns >= w of L and X are
-// zero except for ones on the diagonal (identity padding), so the products
-// need no edge tests.  D is destroyed; `tmp` is a scratch tile (64 x FLD).
-
-// 8 x 8 base case by warp 0, lanes 0..7 holding rows in registers
-// (not inlined: one copy of the code serves every call site, which keeps the
-// recursion's instruction footprint small)
-__device__ __noinline__ void chol_inv8(double *D, double *L, double *X, int w, double pivtol,
-                                       int *status,
-                       int colbase, bool record) {
-    if (threadIdx.x >= 32) return;
-    const unsigned full = 0xffffffffu;
-    const int i = threadIdx.x & 7;
-    const bool act = threadIdx.x < 8;
-    double a[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) a[k] = (i < w && k <= i) ? D[k * FLD + i] : (k == i ? 1.0 : 0.0);
-    double myr = 1.0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        double d = __shfl_sync(full, a[j], j);
-        if (!(d > pivtol)) {
-            if (record && act && i == 0 && j < w) atomicCAS(status, 0, colbase + j + 1);
-            d = 1.0;
-        }
-        const double rl = rsqrt(d);
-        const double lij = (i > j) ? a[j] * rl : (i == j ? d * rl : 0.0);
-        a[j] = lij;
-        if (i == j) myr = rl;
-#pragma unroll
-        for (int k = j + 1; k < 8; k++) {
-            const double lkj = __shfl_sync(full, lij, k);
-            if (k <= i) a[k] -= lij * lkj;
-        }
-    }
-    double x[8];
-#pragma unroll
-    for (int c = 0; c < 8; c++) x[c] = (c == i) ? myr : 0.0;
-#pragma unroll
-    for (int t = 0; t < 7; t++) {
-#pragma unroll
-        for (int c = 0; c <= t; c++) {
-            const double xtc = __shfl_sync(full, x[c], t);
-            if (i > t) x[c] -= a[t] * xtc;
-        }
-        if (i == t + 1)
-#pragma unroll
-            for (int c = 0; c <= t; c++) x[c] *= myr;
-    }
-    if (act)
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            L[k * FLD + i] = a[k];
-            X[k * FLD + i] = x[k];
-        }
-}
-
-// C (h x h) = sum_k A(i, k) B'(k, j) over k < h, for the four small products
-// of the recursion; each thread computes h*h/128 (or one) outputs.
-// mode 0: C = A B^T (A, B both stored row-index-first, i.e. B(j, k))
-// mode 1: C = A B   (B(k, j))
-template <int H, int MODE>
-__device__ __noinline__ void small_mm(const double *A, const double *B, double *C, double alpha,
-                                      bool accumulate) {
-    constexpr int NOUT = H * H;
-    for (int o = threadIdx.x; o < NOUT; o += blockDim.x) {
-        const int i = o % H, j = o / H;
-        double acc = 0.0;
-#pragma unroll
-        for (int k = 0; k < H; k++)
-            acc += A[k * FLD + i] * (MODE == 0 ? B[k * FLD + j] : B[j * FLD + k]);
-        C[j * FLD + i] = accumulate ? C[j * FLD + i] + alpha * acc : alpha * acc;
-    }
-}
-
-template <int N>
-SPX_DEV void chol_inv_rec(double *D, double *L, double *X, double *tmp, int w, double pivtol,
-                          int *status, int colbase, bool record) {
-    if constexpr (N == 8) {
-        chol_inv8(D, L, X, w, pivtol, status, colbase, record);
-        __syncthreads();
-    } else {
-        constexpr int H = N / 2;
-        const int w0 = min(w, H), w1 = max(w - H, 0);
-        chol_inv_rec<H>(D, L, X, tmp, w0, pivtol, status, colbase, record);
-        if (w1 == 0) {
-            // nothing left to factor: identity padding for the second half
-            for (int t = threadIdx.x; t < H * H; t += blockDim.x) {
-                const int i = t % H, j = t / H;
-                L[(H + j) * FLD + i] = 0.0;
-                X[(H + j) * FLD + i] = 0.0;
-                L[j * FLD + H + i] = 0.0;
-                X[j * FLD + H + i] = 0.0;
-                L[(H + j) * FLD + H + i] = (i == j) ? 1.0 : 0.0;
-                X[(H + j) * FLD + H + i] = (i == j) ? 1.0 : 0.0;
-            }
-            __syncthreads();
-            return;
-        }
-        // off-diagonal blocks of L and X above the diagonal stay zero
-        for (int t = threadIdx.x; t < H * H; t += blockDim.x) {
-            const int i = t % H, j = t / H;
-            L[(H + j) * FLD + i] = 0.0;
-            X[(H + j) * FLD + i] = 0.0;
-        }
-        small_mm<H, 0>(D + H, X, L + H, 1.0, false);               // L10 = A10 X00^T
-        __syncthreads();
-        small_mm<H, 0>(L + H, L + H, D + H * FLD + H, -1.0, true); // A11 -= L10 L10^T
-        small_mm<H, 1>(L + H, X, tmp, 1.0, false);                 // T = L10 X00
-        __syncthreads();
-        chol_inv_rec<H>(D + H * FLD + H, L + H * FLD + H, X + H * FLD + H, tmp + H * FLD, w1,
-                        pivtol, status, colbase + H, record);
-        small_mm<H, 1>(X + H * FLD + H, tmp, X + H, -1.0, false);  // X10 = -X11 T
-        __syncthreads();
-    }
-}
-
-// Panel step kb of a front, in two kernels that run on separate streams of
-// the factor graph.  mf_diag64 (one block per front, task = (s, kb, 0, 0)):
-// Cholesky and inverse of the updated diagonal tile kb; inv(L_kk) goes to G
-// (only inv(L_kk) is kept: nothing later reads a diagonal tile of L).  It
-// needs only the update of that one tile by step kb-1, so it runs beside the
-// rest of that step's trailing update.
-__global__ void __launch_bounds__(kGThreads)
-mf_diag64(const int4 *__restrict__ tasks, Sym y, Real *__restrict__ F, Real *__restrict__ G,
-          const double *__restrict__ params, int *status) {
-    extern __shared__ double fsm[];
-    double *Ds = fsm, *Ls = fsm + kFTileDoubles, *Xs = fsm + 2 * kFTileDoubles;
-    double *Ts = fsm + 3 * kFTileDoubles;
-    if (*(volatile int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, kb = tk.y;
-    const Front f = front_of<FT>(y, s);
-    int ka, kz;
-    tile_range<FT>(f, kb, ka, kz);
-    const int w = kz - ka;
-    ftile_load_lower(Ds, F + f.fptr, f.r, ka, w);
-    tiles_ready<Real>(Ds);
-    chol_inv_rec<64>(Ds, Ls, Xs, Ts, w, params[1], status, f.first + ka, true);
-    Real *Gs = G + f.gptr;
-    for (int t = threadIdx.x; t < FT * FT; t += blockDim.x) {
-        const int i = t & (FT - 1), j = t >> 6;
-        if (i < w && j <= i)
-            Gs[(int64_t)(ka + i) + (int64_t)(ka + j) * f.ldg] = (Real)Xs[j * FLD + i];
-    }
-}
-
-// mf_rows64 (task = (s, I0, nI, kb)): the tiles I0 .. I0+nI-1 below the
-// diagonal of column block kb, L_Ik = F_Ik inv(L_kk)^T, with inv(L_kk) read
-// back from G.  A large front's tiles get a block each, a small front's
-// share one; each tile is loaded while the block works on the one before.
-__global__ void __launch_bounds__(kGThreads)
-mf_rows64(const int4 *__restrict__ tasks, Sym y, Real *__restrict__ F,
-          const Real *__restrict__ G, int *status) {
-    extern __shared__ double fsm[];
-    double *Xs = fsm, *Ps = fsm + kFTileDoubles, *Ds = fsm + 2 * kFTileDoubles;
-    if (*(volatile int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, I0 = tk.y, nI = tk.z, kb = tk.w;
-    const Front f = front_of<FT>(y, s);
-    int ka, kz;
-    tile_range<FT>(f, kb, ka, kz);
-    const int w = kz - ka;
-    Real *Fs = F + f.fptr;
-    auto load_tile = [&](double *buf, int I) {
-        int ra, rb;
-        tile_range<FT>(f, I, ra, rb);
-        ftile_load(buf, Fs, f.r, ra, rb - ra, ka, w);
-    };
-    ftile_load_lower(Xs, G + f.gptr, f.ldg, ka, w);
-    load_tile(Ps, I0);
-    cp_commit();
-    double *cur = Ps, *spare = Ds;
-    for (int I = I0; I < I0 + nI; I++) {
-        if (I + 1 < I0 + nI) load_tile(spare, I + 1);
-        cp_commit();
-        cp_wait_all_but_last();      // inv(L_kk) and tile I are in
-        if constexpr (!std::is_same<Real, double>::value) {
-            if (I == I0) tile_widen<Real>(Xs);
-            tile_widen<Real>(cur);
-            __syncthreads();
-        }
-        int ra, rb;
-        tile_range<FT>(f, I, ra, rb);
-        const int h = rb - ra;
-        Acc acc;
-        acc_zero(acc);
-        warp_mma<true>(acc, cur, Xs, (w + 3) & ~3, h, w);
-        acc_store<false>(acc, Fs, f.r, ra, h, ka, w, 1.0, false);
-        __syncthreads();
-        double *t = cur; cur = spare; spare = t;
-    }
-}
-
-// ---- FP32 trailing update on the TF32 tensor cores (mixed precision) --
-// mma.sync m16n8k8 tf32 with FP32 accumulation; every operand is split into
-// a TF32 head and a TF32 tail (x = hi + lo) and the product is taken as
-// hi*hi + hi*lo + lo*hi, which keeps FP32 accuracy.  Tiles are FP32 in
-// shared memory with a leading dimension of 72 floats (conflict-free
-// fragment reads).
-constexpr int FLDF = 72;
-
-SPX_DEV void ftile_load_f32(float *s, const float *M, int64_t ld, int ra, int h, int ca, int w) {
-#pragma unroll 8
-    for (int q = 0; q < FT * FT / kGThreads; q++) {
-        const int t = threadIdx.x + q * kGThreads;
-        const int i = t & (FT - 1), j = t >> 6;
-        const bool v = (i < h && j < w);
-        cp_async4(s + j * FLDF + i, v ? M + (int64_t)(ra + i) + (int64_t)(ca + j) * ld : M, v);
-    }
-}
-SPX_DEV uint32_t tf32_of(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
-}
-SPX_DEV void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
-    hi = tf32_of(x);
-    lo = tf32_of(x - __uint_as_float(hi));
-}
-SPX_DEV void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-        "{%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// F_IJ -= L_Ik L_Jk^T on FP32 tiles: warp tile 32 x 32 = 2 x 4 fragments.
-// The output tile is staged in Cs with the operands, so the subtraction does
-// not wait on global loads after the products.
-SPX_DEV void update_tile_f32(float *Fs, int ld, int ra, int h, int ca, int w, int ka, int kw,
-                             float *As, float *Bs, float *Cs) {
-    ftile_load_f32(As, Fs, ld, ra, h, ka, kw);
-    ftile_load_f32(Bs, Fs, ld, ca, w, ka, kw);
-    ftile_load_f32(Cs, Fs, ld, ra, h, ca, w);
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int wid = threadIdx.x >> 5, m0 = (wid & 1) * 32, n0 = (wid >> 1) * 32;
-    if (m0 >= h || n0 >= w) return;
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
-    const int kw8 = (kw + 7) & ~7;
-    for (int k = 0; k < kw8; k += 8) {
-        uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int r = m0 + 16 * i + g;
-            split_tf32(As[(k + t) * FLDF + r], ah[i][0], al[i][0]);
-            split_tf32(As[(k + t) * FLDF + r + 8], ah[i][1], al[i][1]);
-            split_tf32(As[(k + t + 4) * FLDF + r], ah[i][2], al[i][2]);
-            split_tf32(As[(k + t + 4) * FLDF + r + 8], ah[i][3], al[i][3]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + 8 * j + g;
-            split_tf32(Bs[(k + t) * FLDF + n], bh[j][0], bl[j][0]);
-            split_tf32(Bs[(k + t + 4) * FLDF + n], bh[j][1], bl[j][1]);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                mma_tf32(acc[i][j], al[i], bh[j]);
-                mma_tf32(acc[i][j], ah[i], bl[j]);
-                mma_tf32(acc[i][j], ah[i], bh[j]);
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int m = m0 + 16 * i + g + 8 * (e >> 1), n = n0 + 8 * j + 2 * t + (e & 1);
-                if (m < h && n < w)
-                    Fs[(int64_t)(ra + m) + (int64_t)(ca + n) * ld] = Cs[n * FLDF + m] - acc[i][j][e];
-            }
-}
-
-// F_IJ -= L_Ik L_Jk^T    task = (s, I, J, kb)
-__global__ void __launch_bounds__(kGThreads)
-mf_update64(const int4 *__restrict__ tasks, Sym y, Real *__restrict__ F, const int *status) {
-    extern __shared__ double fsm[];
-    if (*(volatile const int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, I = tk.y, J = tk.z, kb = tk.w;
-    const Front f = front_of<FT>(y, s);
-    int ra, rb, ca, cb, ka, kz;
-    tile_range<FT>(f, I, ra, rb);
-    tile_range<FT>(f, J, ca, cb);
-    tile_range<FT>(f, kb, ka, kz);
-    const int h = rb - ra, w = cb - ca, kw = kz - ka;
-    Real *Fs = F + f.fptr;
-    if constexpr (std::is_same<Real, float>::value) {
-        float *As = reinterpret_cast<float *>(fsm), *Bs = As + FT * FLDF, *Cs = Bs + FT * FLDF;
-        update_tile_f32(reinterpret_cast<float *>(Fs), f.r, ra, h, ca, w, ka, kw, As, Bs, Cs);
-    } else {
-        // the output tile is staged with the operands, so the subtraction
-        // does not wait on global loads after the products
-        double *As = fsm, *Bs = fsm + kFTileDoubles, *Cs = fsm + 2 * kFTileDoubles;
-        ftile_load(As, Fs, f.r, ra, h, ka, kw);
-        ftile_load(Bs, Fs, f.r, ca, w, ka, kw);
-        ftile_load(Cs, Fs, f.r, ra, h, ca, w);
-        cp_wait();
-        Acc acc;
-        acc_zero(acc);
-        warp_mma<true>(acc, As, Bs, (kw + 3) & ~3, h, w);
-        acc_sub_store(acc, Cs, Fs, f.r, ra, h, ca, w);
-    }
-}
-
-// inv(L11) by recursive doubling over tile blocks.  After step l every
-// diagonal block of 2^l tiles is inverted; step l joins blocks A = [A0, C0)
-// and C = [C0, C1) (C0 = A0 + 2^l) through
-//   T = L_CA X_A          (mf_inv_t64: T lands in the unused upper part of F)
-//   X_CA = -X_C T         (mf_inv_x64)
-// task = (s, i, j, l): output tile (i, j), i in C, j in A.
-__global__ void __launch_bounds__(kGThreads)
-mf_inv_t64(const int4 *__restrict__ tasks, Sym y, Real *__restrict__ F,
-           const Real *__restrict__ G, const int *status) {
-    extern __shared__ double fsm[];
-    double *As = fsm, *Bs = fsm + kFTileDoubles;
-    if (*(volatile const int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, i = tk.y, j = tk.z, l = tk.w;
-    const Front f = front_of<FT>(y, s);
-    const int C0 = (j >> (l + 1) << (l + 1)) + (1 << l);
-    int ra, rb, ca, cb;
-    tile_range<FT>(f, i, ra, rb);
-    tile_range<FT>(f, j, ca, cb);
-    const int h = rb - ra, w = cb - ca;
-    Real *Fs = F + f.fptr;
-    const Real *Gs = G + f.gptr;
-    Acc acc;
-    acc_zero(acc);
-    for (int k = j; k < C0; k++) {
-        int ka, kz;
-        tile_range<FT>(f, k, ka, kz);
-        const int kw = kz - ka;
-        ftile_load(As, Fs, f.r, ra, h, ka, kw);      // L_ik
-        ftile_load(Bs, Gs, f.ldg, ka, kw, ca, w);    // X_kj
-        tiles_ready<Real>(As, Bs);
-        warp_mma<false>(acc, As, Bs, (kw + 3) & ~3, h, w);
-        __syncthreads();
-    }
-    // T_ij is kept at tile (j, i) of F: strictly upper, never used otherwise
-    acc_store<true>(acc, Fs, f.r, ra, h, ca, w, 1.0, false);
-}
-
-__global__ void __launch_bounds__(kGThreads)
-mf_inv_x64(const int4 *__restrict__ tasks, Sym y, const Real *__restrict__ F,
-           Real *__restrict__ G, const int *status) {
-    extern __shared__ double fsm[];
-    double *As = fsm, *Bs = fsm + kFTileDoubles;
-    if (*(volatile const int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, i = tk.y, j = tk.z, l = tk.w;
-    const Front f = front_of<FT>(y, s);
-    const int C0 = (j >> (l + 1) << (l + 1)) + (1 << l);
-    int ra, rb, ca, cb;
-    tile_range<FT>(f, i, ra, rb);
-    tile_range<FT>(f, j, ca, cb);
-    const int h = rb - ra, w = cb - ca;
-    const Real *Fs = F + f.fptr;
-    Real *Gs = G + f.gptr;
-    Acc acc;
-    acc_zero(acc);
-    for (int k = C0; k <= i; k++) {
-        int ka, kz;
-        tile_range<FT>(f, k, ka, kz);
-        const int kw = kz - ka;
-        ftile_load(As, Gs, f.ldg, ra, h, ka, kw);    // X_ik
-        ftile_load_t(Bs, Fs, f.r, ka, kw, ca, w);    // T_kj, stored transposed at tile (j, k)
-        tiles_ready<Real>(As, Bs);
-        warp_mma<false>(acc, As, Bs, (kw + 3) & ~3, h, w);
-        __syncthreads();
-    }
-    acc_store<false>(acc, Gs, f.ldg, ra, h, ca, w, -1.0, false);
-}
-
-// W_IJ = sum_{K=J}^{nkb-1} L_IK X_KJ   (I a tile of the rows below the pivots)
-__global__ void __launch_bounds__(kGThreads)
-mf_wmul64(const int4 *__restrict__ tasks, Sym y, const Real *__restrict__ F,
-          Real *__restrict__ G, const int *status) {
-    extern __shared__ double fsm[];
-    double *As = fsm, *Bs = fsm + kFTileDoubles;
-    if (*(volatile const int *)status) return;
-    const int4 tk = tasks[blockIdx.x];
-    const int s = tk.x, I = tk.y, J = tk.z;
-    const Front f = front_of<FT>(y, s);
-    int ra, rb, ca, cb;
-    tile_range<FT>(f, I, ra, rb);
-    tile_range<FT>(f, J, ca, cb);
-    const int h = rb - ra, w = cb - ca;
-    const Real *Fs = F + f.fptr;
-    Real *Gs = G + f.gptr;
-    Acc acc;
-    acc_zero(acc);
-    for (int k = J; k < f.nkb; k++) {
-        int ka, kz;
-        tile_range<FT>(f, k, ka, kz);
-        const int kw = kz - ka;
-        ftile_load(As, Fs, f.r, ra, h, ka, kw);
-        ftile_load(Bs, Gs, f.ldg, ka, kw, ca, w);
-        tiles_ready<Real>(As, Bs);
-        warp_mma<false>(acc, As, Bs, (kw + 3) & ~3, h, w);
-        __syncthreads();
-    }
-    acc_store<false>(acc, Gs, f.ldg, ra, h, ca, w, 1.0, false);
-}
-
 
 // ---------------------------------------------------------------- solve --
 // The whole solve pair is one persistent kernel that pulls tasks from an
@@ -1597,6 +696,7 @@ __global__ void __launch_bounds__(kSThreads, 2) mf_solve_sf(SolveArgs a) {
     solve_warp_tasks(a, a.wtasks + a.nfw, a.nbw, a.sync + 1 + 4 * a.ns, ws[wid]);
 }
 
+#include "mf_factor.cuh"
 #include "mf_block_solve.cuh"
 
 static size_t solve_smem_bytes() {
@@ -1612,6 +712,151 @@ struct SNodeH {
 struct STaskH {
     int kind, s, I, J, chunk, boff, bn, pad;
 };
+
+struct FNodeH {
+    int first, c, r, ldg, parent, nchild, child0, expect;
+    long long fptr, uptr, gptr, g0;
+    int flag0, nkb, nt, unused, pad[4];
+};
+struct FChildH {
+    long long uptr, relmap;
+    int cbnd, nb, pad[2];
+};
+struct FTaskH { int kind, s, I, J; };
+static_assert(sizeof(FNodeH) == sizeof(FNode), "factor node layout");
+static_assert(sizeof(FChildH) == sizeof(FChild), "factor child layout");
+static_assert(sizeof(FTaskH) == sizeof(FTask), "factor task layout");
+
+// The factor's nodes, tile storage (in Reals) and task queue.
+//
+// A task's key is an estimate (us) of the path from it to the end of the
+// root: a column block of a front's diagonal chain costs kStep, and a front
+// kFront for its assembly and hand-over.  Tasks run in decreasing key order,
+// equal keys in the order they were made, which puts every task after the
+// ones it waits for: a front starts below its children's update tiles, a
+// column block below the one before it, rows below their diagonal tile.
+// Inverse tiles follow two column blocks behind the chain; W tiles, which no
+// factor task waits for, fill the middle of the parent's chain.
+static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
+                              std::vector<FNodeH> &node, std::vector<FChildH> &child,
+                              std::vector<int32_t> &cbnd, std::vector<FTaskH> &tasks,
+                              int64_t *storage, int64_t *nflags) {
+    constexpr int kStep = 15, kFront = 12, kRes = 4;
+    const int32_t ns = S.nsuper;
+    int64_t off = 0, nfl = 0;
+    std::vector<int32_t> start(ns, 0);           // key of a front's first task
+    auto r4 = [](int64_t v) { return (v + 3) & ~(int64_t)3; };
+    auto is_small = [&](int32_t s) { return node[s].nkb == 1 && node[s].nt <= 2; };
+    for (int32_t s = 0; s < ns; s++) {
+        FNodeH &m = node[s];
+        m = FNodeH();
+        m.first = S.sfirst[s];
+        m.c = S.sfirst[s + 1] - S.sfirst[s];
+        m.r = (int)(S.rowptr[s + 1] - S.rowptr[s]);
+        m.ldg = (m.r + kLdgA - 1) & ~(kLdgA - 1);
+        m.parent = S.sparent[s];
+        m.nchild = S.child_ptr[s + 1] - S.child_ptr[s];
+        m.child0 = S.child_ptr[s];
+        m.gptr = gptr[s];
+        m.g0 = S.rowptr[s];
+        m.nkb = (m.c + FT - 1) / FT;
+        const int64_t nb = m.r - m.c, nu = (nb + FT - 1) / FT, nkb = m.nkb;
+        m.nt = (int)(nkb + nu);
+        const int64_t wc4 = r4(m.c - (nkb - 1) * FT);
+        m.fptr = off;
+        if (!is_small(s)) {
+            // lower pivot tiles, then the transposed inverse's tiles
+            off += (int64_t)FT * FT * ((nkb - 1) * m.nt - (nkb - 1) * (nkb - 2) / 2) + FT * wc4 * (nu + 1);
+            off += (int64_t)FT * FT * (nkb * (nkb - 1) / 2) + FT * wc4 * nkb;
+            m.flag0 = (int)nfl;
+            nfl += nkb * m.nt + nkb * nkb;
+        }
+        m.uptr = off;
+        if (nu > 0) {
+            const int64_t wl4 = r4(nb - (nu - 1) * FT);
+            off += (int64_t)FT * FT * ((nu - 1) * nu - (nu - 1) * (nu - 2) / 2) + FT * wl4;
+        }
+    }
+    for (int32_t s = ns - 1; s >= 0; s--) {
+        const FNodeH &m = node[s];
+        start[s] = kRes * (kFront + kStep * m.nkb) + (m.parent < 0 ? 0 : start[m.parent]);
+    }
+    int64_t ntask = 0, nbnd = 0;
+    for (int32_t s = 0; s < ns; s++) {
+        const FNodeH &m = node[s];
+        const int64_t nu = m.nt - m.nkb, nkb = m.nkb;
+        ntask += is_small(s) ? 1 : (int64_t)m.nt * (m.nt + 1) / 2 + nkb * (nkb - 1) / 2 + nu * nkb;
+        if (m.parent >= 0) {
+            node[m.parent].expect += is_small(s) ? nu : nu * (nu + 1) / 2;
+            nbnd += node[m.parent].nt + 1;
+        }
+    }
+    // the children's records and their bounds per 64-row tile of the parent
+    cbnd.reserve(nbnd);
+    for (int32_t p = 0; p < ns; p++)
+        for (int32_t q = S.child_ptr[p]; q < S.child_ptr[p + 1]; q++) {
+            const int32_t ch = S.child_list[q];
+            FChildH &c = child[q];
+            c = FChildH();
+            c.uptr = node[ch].uptr;
+            c.relmap = S.rowptr[ch] + node[ch].c;
+            c.nb = node[ch].r - node[ch].c;
+            c.cbnd = (int)cbnd.size();
+            const int32_t *rm = S.relmap + c.relmap;
+            const FNodeH &m = node[p];
+            int32_t at = 0;
+            for (int I = 0; I <= m.nt; I++) {
+                const int row = I == m.nt ? m.r : I < m.nkb ? I * FT : m.c + (I - m.nkb) * FT;
+                at = (int32_t)(std::lower_bound(rm + at, rm + c.nb, row) - rm);
+                cbnd.push_back(at);
+            }
+        }
+    std::vector<FTaskH> t;
+    std::vector<int32_t> key;
+    t.reserve(ntask);
+    key.reserve(ntask);
+    int32_t kmin = 0, kmax = 0;
+    auto emit = [&](int kind, int s, int I, int J, int k) {
+        t.push_back({kind, s, I, J});
+        key.push_back(k);
+        kmin = std::min(kmin, k);
+        kmax = std::max(kmax, k);
+    };
+    for (int32_t s = 0; s < ns; s++) {
+        const FNodeH &m = node[s];
+        if (is_small(s)) {
+            emit(FK_SMALL, s, 0, 0, start[s]);
+            continue;
+        }
+        const int up = m.parent < 0 ? 0 : start[m.parent];
+        const int tp = m.parent < 0 ? 0 : kRes * (kFront + kStep * node[m.parent].nkb);
+        for (int J = 0; J < m.nkb; J++) {
+            emit(FK_DIAG, s, J, J, start[s] - kRes * kStep * J);
+            for (int I = J + 1; I < m.nt; I++) emit(FK_ROWS, s, I, J, start[s] - kRes * (kStep * J + 4));
+        }
+        for (int J = m.nkb; J < m.nt; J++)
+            for (int I = J; I < m.nt; I++) emit(FK_SCHUR, s, I, J, up + kRes * 8);
+        for (int i = 1; i < m.nkb; i++)
+            for (int j = 0; j < i; j++) emit(FK_INV, s, i, j, start[s] - kRes * (kStep * i + 20));
+        for (int J = 0; J < m.nkb; J++)
+            for (int I = m.nkb; I < m.nt; I++) emit(FK_WMUL, s, I, J, up - kRes * 2 - tp / 2);
+    }
+    const int64_t range = (int64_t)kmax - kmin + 1;
+    tasks.resize(t.size());
+    if (range <= 4 * (int64_t)t.size() + 65536) {
+        std::vector<int32_t> cnt(range + 1, 0);
+        for (int32_t k : key) cnt[kmax - k + 1]++;
+        for (int64_t q = 0; q < range; q++) cnt[q + 1] += cnt[q];
+        for (size_t i = 0; i < t.size(); i++) tasks[cnt[kmax - key[i]]++] = t[i];
+    } else {
+        std::vector<int32_t> ord(t.size());
+        for (size_t i = 0; i < t.size(); i++) ord[i] = (int32_t)i;
+        std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key[x] > key[y]; });
+        for (size_t i = 0; i < t.size(); i++) tasks[i] = t[ord[i]];
+    }
+    *storage = off;
+    *nflags = nfl;
+}
 
 template <class Tp>
 static int dmalloc(Tp **p, size_t cnt, cudaStream_t st) {
@@ -1644,37 +889,20 @@ static int dupload(Tp **p, const Tp *h, size_t cnt, cudaStream_t st) {
 template <> MultifrontalPlanT<Real>::~MultifrontalPlanT() { release(0); }
 
 template <> void MultifrontalPlanT<Real>::release(cudaStream_t st) {
-    if (fgraph_) { cudaGraphExecDestroy(fgraph_); fgraph_ = nullptr; }
-    fgraph_val_ = nullptr;
-    direct_val_ = nullptr;
-    for (auto &e : fev_)
-        if (e) { cudaEventDestroy(e); e = nullptr; }
-    if (fside_) { cudaStreamDestroy(fside_); fside_ = nullptr; }
-    if (d_params_) { cudaFreeAsync(d_params_, st); d_params_ = nullptr; }
-    void *ptrs[] = {d_cbnd_, d_cbnd_ptr_, d_perm_, d_sfirst_, d_rows_, d_relmap_, d_child_ptr_, d_child_list_,
-                    d_rowptr_, d_frontptr_, d_gptr_, d_uptr_, d_acolptr_, d_atpos_, d_asrc_,
-                    d_tasks_, d_front_, d_G_, d_u_, d_yf_, d_x_, d_status_, d_meta_,
-                    d_stask_, d_bundle_, d_cptr_, d_cidx_, d_chunks_, d_fpart_, d_bpart_,
-                    d_cnt_, d_sync_, d_byf_, d_bx_, d_bu_, d_bfp_, d_bbp_};
-    for (void *p : ptrs)
-        if (p) cudaFreeAsync(p, st);
-    d_byf_ = d_bx_ = d_bu_ = d_bfp_ = d_bbp_ = nullptr;
+    void **ptrs[] = {(void **)&d_params_, (void **)&d_perm_, (void **)&d_rows_, (void **)&d_relmap_,
+                     (void **)&d_cbnd_, (void **)&d_fnode_, (void **)&d_fchild_, (void **)&d_ftask_,
+                     (void **)&d_fsync_, (void **)&d_acolptr_, (void **)&d_atpos_, (void **)&d_asrc_,
+                     (void **)&d_front_, (void **)&d_G_, (void **)&d_u_, (void **)&d_yf_,
+                     (void **)&d_x_, (void **)&d_meta_, (void **)&d_stask_, (void **)&d_bundle_,
+                     (void **)&d_cptr_, (void **)&d_cidx_, (void **)&d_chunks_, (void **)&d_fpart_,
+                     (void **)&d_bpart_, (void **)&d_cnt_, (void **)&d_sync_, (void **)&d_byf_,
+                     (void **)&d_bx_, (void **)&d_bu_, (void **)&d_bfp_, (void **)&d_bbp_};
+    for (void **p : ptrs)
+        if (*p) {
+            cudaFreeAsync(*p, st);
+            *p = nullptr;
+        }
     bw_ = 0;
-    d_perm_ = d_sfirst_ = d_rows_ = d_relmap_ = d_child_ptr_ = d_child_list_ = nullptr;
-    d_cbnd_ = nullptr;
-    d_cbnd_ptr_ = nullptr;
-    d_rowptr_ = d_frontptr_ = d_gptr_ = d_uptr_ = nullptr;
-    d_acolptr_ = d_atpos_ = d_asrc_ = nullptr;
-    d_tasks_ = nullptr;
-    d_bundle_ = d_cptr_ = d_cidx_ = d_chunks_ = nullptr;
-    d_meta_ = nullptr;
-    d_stask_ = nullptr;
-    d_fpart_ = d_bpart_ = nullptr;
-    d_cnt_ = d_sync_ = nullptr;
-    d_front_ = nullptr;
-    d_G_ = nullptr;
-    d_u_ = d_yf_ = d_x_ = nullptr;
-    d_status_ = nullptr;
 }
 
 template <> int64_t MultifrontalPlanT<Real>::solve_bytes() const {
@@ -1690,8 +918,6 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
     ns_ = S.nsuper;
     nlevels_ = S.nlevels;
     flops_ = S.flops;
-    front_total_ = S.front_total;
-    max_rows_ = S.max_rows;
     nrows_total_ = S.rowptr[ns_];
     const int32_t n = n_, ns = ns_;
     try {
@@ -1711,8 +937,10 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         std::vector<int32_t> acolptr(n + 1, 0);
         std::vector<int32_t> atpos, asrc;
         std::vector<int32_t> cptr(nrows_total_ + 1, 0), cidx;
-        std::vector<int64_t> cbnd_ptr(ns + 1, 0);
         std::vector<int32_t> cbnd;
+        std::vector<FNodeH> fnode(ns);
+        std::vector<FChildH> fchild(S.child_ptr[ns]);
+        std::vector<FTaskH> ftask;
         TaskGroup side(rowptr[n] >= (1 << 17));
         side.run([&] {
             // assembly entries: for new column j, the entries of A's column
@@ -1731,7 +959,7 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
             for (int32_t j = 0; j < n; j++) acolptr[j + 1] += acolptr[j];
             atpos.resize(acolptr[n]);
             asrc.resize(acolptr[n]);
-            parallel_ranges(ns, 2048, [&](int64_t lo, int64_t hi) {
+            parallel_ranges(ns, 128, [&](int64_t lo, int64_t hi) {
                 std::vector<int32_t> pos(n, -1);
                 std::vector<std::pair<int32_t, int32_t>> tmp;
                 for (int64_t s = lo; s < hi; s++) {
@@ -1778,159 +1006,9 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
                     }
             }
         });
-        side.run([&] {
-            // child tile bounds for the assembly (32-row tiles of the parent)
-            for (int32_t ch = 0; ch < ns; ch++) {
-                const int p = S.sparent[ch];
-                cbnd_ptr[ch] = (int64_t)cbnd.size();
-                if (p < 0) continue;
-                const int rp = (int)(S.rowptr[p + 1] - S.rowptr[p]);
-                const int cp = S.sfirst[p + 1] - S.sfirst[p];
-                const int nkb = (cp + T - 1) / T, ntp = nkb + (rp - cp + T - 1) / T;
-                const int cch = S.sfirst[ch + 1] - S.sfirst[ch];
-                const int32_t *rm = S.relmap + S.rowptr[ch] + cch;
-                const int nb = (int)(S.rowptr[ch + 1] - S.rowptr[ch]) - cch;
-                for (int I = 0; I <= ntp; I++) {
-                    const int start = (I == ntp) ? rp : (I < nkb ? I * T : cp + (I - nkb) * T);
-                    cbnd.push_back((int32_t)(std::lower_bound(rm, rm + nb, start) - rm));
-                }
-            }
-            cbnd_ptr[ns] = (int64_t)cbnd.size();
-        });
-        // tile task lists, level by level (on a side thread: nothing below
+        // factor nodes, tile storage and the tile task queue (nothing below
         // reads them before the uploads)
-        std::vector<int4> tasks;
-        side.run([&] {
-            launches_.clear();
-            use_side_ = false;
-            auto emit = [&](int kind, size_t before) {
-                if (tasks.size() > before)
-                    launches_.push_back({kind, (int64_t)before, (int64_t)(tasks.size() - before)});
-            };
-            auto is_tiny = [&](int s) { return S.rowptr[s + 1] - S.rowptr[s] <= T; };
-            for (int l = 0; l < S.nlevels; l++) {
-                const int32_t q0 = S.level_ptr[l], q1 = S.level_ptr[l + 1];
-                int nkbmax = 0;
-                {
-                    size_t bt = tasks.size();
-                    for (int32_t q = q0; q < q1; q++)
-                        if (is_tiny(S.level_sup[q])) tasks.push_back(make_int4(S.level_sup[q], 0, 0, 0));
-                    emit(MF_TINY, bt);
-                }
-                size_t b = tasks.size();
-                for (int32_t q = q0; q < q1; q++) {
-                    const int s = S.level_sup[q];
-                    if (is_tiny(s)) continue;
-                    const int r = (int)(S.rowptr[s + 1] - S.rowptr[s]);
-                    const int c = S.sfirst[s + 1] - S.sfirst[s];
-                    const int nkb = (c + T - 1) / T, nt = nkb + (r - c + T - 1) / T;
-                    nkbmax = std::max(nkbmax, nkb);
-                    for (int I = 0; I < nt; I++)
-                        for (int J = 0; J <= I; J++) tasks.push_back(make_int4(s, I, J, 0));
-                }
-                emit(MF_ASSEMBLE, b);
-                // factor steps on 64-tiles: diagonal tile kb, the tiles below
-                // it, then the right-looking update of the trailing tiles,
-                // Schur complement included
-                auto geo = [&](int s, int &r, int &c, int &nkb, int &nt) {
-                    r = (int)(S.rowptr[s + 1] - S.rowptr[s]);
-                    c = S.sfirst[s + 1] - S.sfirst[s];
-                    nkb = (c + FT - 1) / FT;
-                    nt = nkb + (r - c + FT - 1) / FT;
-                };
-                nkbmax = 0;
-                for (int32_t q = q0; q < q1; q++) {
-                    const int s = S.level_sup[q];
-                    if (is_tiny(s)) continue;
-                    int r, c, nkb, nt;
-                    geo(s, r, c, nkb, nt);
-                    nkbmax = std::max(nkbmax, nkb);
-                }
-                // step kb: the diagonal tile (mf_diag64), the tiles below it
-                // (mf_rows64), the update of column block kb+1 (the next
-                // diagonal tile depends only on it), then the rest of the
-                // trailing update, which runs beside the next diagonal step.
-                // These four launches are recorded even when empty: they carry
-                // the cross-stream ordering of the factor graph.
-                auto emit_always = [&](int kind, size_t before) {
-                    launches_.push_back({kind, (int64_t)before, (int64_t)(tasks.size() - before)});
-                };
-                if (nkbmax >= 2) use_side_ = true;
-                for (int kb = 0; kb < nkbmax; kb++) {
-                    size_t b0 = tasks.size();
-                    for (int32_t q = q0; q < q1; q++) {
-                        const int s = S.level_sup[q];
-                        if (is_tiny(s)) continue;
-                        int r, c, nkb, nt;
-                        geo(s, r, c, nkb, nt);
-                        if (nkb > kb) tasks.push_back(make_int4(s, kb, 0, 0));
-                    }
-                    emit_always(MF_DIAG, b0);
-                    b0 = tasks.size();
-                    for (int32_t q = q0; q < q1; q++) {
-                        const int s = S.level_sup[q];
-                        if (is_tiny(s)) continue;
-                        int r, c, nkb, nt;
-                        geo(s, r, c, nkb, nt);
-                        if (nkb <= kb || nt - kb <= 1) continue;
-                        // a front with few tiles left: one block; else one per tile
-                        if (nt - kb - 1 <= kPanelGroup) tasks.push_back(make_int4(s, kb + 1, nt - kb - 1, kb));
-                        else
-                            for (int I = kb + 1; I < nt; I++) tasks.push_back(make_int4(s, I, 1, kb));
-                    }
-                    emit_always(MF_ROWS, b0);
-                    b0 = tasks.size();
-                    for (int32_t q = q0; q < q1; q++) {
-                        const int s = S.level_sup[q];
-                        if (is_tiny(s)) continue;
-                        int r, c, nkb, nt;
-                        geo(s, r, c, nkb, nt);
-                        if (nkb <= kb) continue;
-                        for (int I = kb + 1; I < nt; I++) tasks.push_back(make_int4(s, I, kb + 1, kb));
-                    }
-                    emit_always(MF_UPD_NEXT, b0);
-                    b0 = tasks.size();
-                    for (int32_t q = q0; q < q1; q++) {
-                        const int s = S.level_sup[q];
-                        if (is_tiny(s)) continue;
-                        int r, c, nkb, nt;
-                        geo(s, r, c, nkb, nt);
-                        if (nkb <= kb) continue;
-                        for (int I = kb + 2; I < nt; I++)
-                            for (int J = kb + 2; J <= I; J++) tasks.push_back(make_int4(s, I, J, kb));
-                    }
-                    emit(MF_UPDATE, b0);
-                }
-                for (int l = 0; (1 << l) < nkbmax; l++) {
-                    const int half = 1 << l;
-                    for (int phase = 0; phase < 2; phase++) {
-                        size_t b0 = tasks.size();
-                        for (int32_t q = q0; q < q1; q++) {
-                            const int s = S.level_sup[q];
-                            if (is_tiny(s)) continue;
-                            int r, c, nkb, nt;
-                            geo(s, r, c, nkb, nt);
-                            for (int A0 = 0; A0 + half < nkb; A0 += 2 * half) {
-                                const int C0 = A0 + half, C1 = std::min(A0 + 2 * half, nkb);
-                                for (int i = C0; i < C1; i++)
-                                    for (int j = A0; j < C0; j++) tasks.push_back(make_int4(s, i, j, l));
-                            }
-                        }
-                        emit(phase == 0 ? MF_INV_T : MF_INV_X, b0);
-                    }
-                }
-                size_t bw = tasks.size();
-                for (int32_t q = q0; q < q1; q++) {
-                    const int s = S.level_sup[q];
-                    if (is_tiny(s)) continue;
-                    int r, c, nkb, nt;
-                    geo(s, r, c, nkb, nt);
-                    for (int I = nkb; I < nt; I++)
-                        for (int J = 0; J < nkb; J++) tasks.push_back(make_int4(s, I, J, 0));
-                }
-                emit(MF_WMUL, bw);
-            }
-        });
+        side.run([&] { plan_factor_tasks(S, gptr.data(), fnode, fchild, cbnd, ftask, &front_total_, &nflags_); });
         // solve: per-supernode metadata and the task queue.  Forward tasks
         // level by level from the leaves (tiles of large supernodes first,
         // then bundles of up to 8 small ones), then backward tasks level by
@@ -2107,21 +1185,18 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         side.wait();
         int rc = 0;
         rc = rc ? rc : dupload(&d_cbnd_, cbnd.data(), cbnd.size(), st);
-        rc = rc ? rc : dupload(&d_cbnd_ptr_, cbnd_ptr.data(), cbnd_ptr.size(), st);
+        rc = rc ? rc : dupload((FNodeH **)&d_fnode_, fnode.data(), fnode.size(), st);
+        rc = rc ? rc : dupload((FChildH **)&d_fchild_, fchild.data(), fchild.size(), st);
+        rc = rc ? rc : dupload((FTaskH **)&d_ftask_, ftask.data(), ftask.size(), st);
+        nftask_ = (int)ftask.size();
+        // tile flags | update tiles finished per parent | queue, status, error
+        rc = rc ? rc : dmalloc(&d_fsync_, (size_t)nflags_ + ns + 3, st);
         rc = rc ? rc : dupload(&d_perm_, S.perm, n, st);
-        rc = rc ? rc : dupload(&d_sfirst_, S.sfirst, ns + 1, st);
         rc = rc ? rc : dupload(&d_rows_, S.rows, (size_t)nrows_total_, st);
         rc = rc ? rc : dupload(&d_relmap_, S.relmap, (size_t)nrows_total_, st);
-        rc = rc ? rc : dupload(&d_child_ptr_, S.child_ptr, ns + 1, st);
-        rc = rc ? rc : dupload(&d_child_list_, S.child_list, ns, st);
-        rc = rc ? rc : dupload(&d_rowptr_, S.rowptr, ns + 1, st);
-        rc = rc ? rc : dupload(&d_frontptr_, S.frontptr, ns + 1, st);
-        rc = rc ? rc : dupload(&d_gptr_, gptr.data(), ns + 1, st);
-        rc = rc ? rc : dupload(&d_uptr_, uptr.data(), ns + 1, st);
         rc = rc ? rc : dupload(&d_acolptr_, acolptr.data(), n + 1, st);
         rc = rc ? rc : dupload(&d_atpos_, atpos.data(), atpos.size(), st);
         rc = rc ? rc : dupload(&d_asrc_, asrc.data(), asrc.size(), st);
-        rc = rc ? rc : dupload(&d_tasks_, tasks.data(), tasks.size(), st);
         {
             std::vector<int32_t> ch;
             ch.insert(ch.end(), fc_base.begin(), fc_base.end());
@@ -2155,26 +1230,21 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         rc = rc ? rc : dmalloc(&d_u_, (size_t)u_total_, st);
         rc = rc ? rc : dmalloc(&d_yf_, (size_t)n, st);
         rc = rc ? rc : dmalloc(&d_x_, (size_t)n, st);
-        rc = rc ? rc : dmalloc(&d_status_, 1, st);
         if (rc) return rc;
         // everything uploaded above comes from host vectors that die here
         if (cudaStreamSynchronize(st) != cudaSuccess) return SPEIGS_ERR_INTERNAL;
-        // persistent grid for the task-queue solve
-        // factor tile kernels stage two or three 64 x 64 tiles
-        cudaFuncSetAttribute(mf_diag64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem);
-        cudaFuncSetAttribute(mf_rows64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
-        cudaFuncSetAttribute(mf_update64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(3 * sizeof(double) * kFTileDoubles));
-        cudaFuncSetAttribute(mf_inv_t64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
-        cudaFuncSetAttribute(mf_inv_x64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
-        cudaFuncSetAttribute(mf_wmul64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
+        // persistent grids
+        int dev = 0, nsm = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        cudaFuncSetAttribute(mf_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FShared));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf_factor, kFThreads, sizeof(FShared));
+        if (per_sm <= 0 || nsm <= 0) return SPEIGS_ERR_INTERNAL;
+        factor_grid_ = nsm * per_sm;
         solve_smem_ = solve_smem_bytes();
         if (solve_smem_ > 48 * 1024)
             cudaFuncSetAttribute(mf_solve_sf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)solve_smem_);
-        int dev = 0, nsm = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf_solve_sf, kSThreads, solve_smem_);
         if (per_sm <= 0 || nsm <= 0) return SPEIGS_ERR_INTERNAL;
         solve_grid_ = nsm * std::min(per_sm, 4);
@@ -2184,65 +1254,6 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
     return 0;
 }
 
-template <> void MultifrontalPlanT<Real>::launch_factor(const double *d_val, cudaStream_t st) {
-    Sym y{d_sfirst_, d_rows_, d_relmap_, d_child_ptr_, d_child_list_, d_rowptr_, d_frontptr_,
-          d_gptr_, d_cbnd_, d_cbnd_ptr_};
-    // with no front of two or more column blocks there is nothing to overlap:
-    // every launch goes on st, in order
-    const bool side = use_side_ && fside_;
-    cudaStream_t sd = side ? fside_ : st;
-    for (const MfLaunch &L : launches_) {
-        const int4 *tk = d_tasks_ + L.off;
-        const unsigned nb = (unsigned)L.count;
-        switch (L.kind) {
-            case MF_ASSEMBLE:
-                mf_assemble<<<nb, kFThreads, 0, st>>>(tk, y, d_front_, d_acolptr_, d_atpos_,
-                                                      d_asrc_, d_val, d_params_, d_status_);
-                if (side) cudaEventRecord(fev_[0], st);
-                break;
-            case MF_TINY:
-                mf_tiny_front<<<(nb + kTinyWarps - 1) / kTinyWarps, 32 * kTinyWarps, 0, st>>>(
-                    tk, (int)nb, y, d_front_, d_G_, d_acolptr_, d_atpos_, d_asrc_, d_val, d_params_,
-                    d_status_);
-                break;
-            case MF_DIAG:
-                // after the update of this diagonal tile (the last record of
-                // fev_[0] on st), beside the rest of the previous update
-                if (side) cudaStreamWaitEvent(sd, fev_[0], 0);
-                if (nb) mf_diag64<<<nb, kGThreads, kPanelSmem, sd>>>(tk, y, d_front_, d_G_,
-                                                                      d_params_, d_status_);
-                break;
-            case MF_ROWS:
-                if (nb) mf_rows64<<<nb, kGThreads, kRowsSmem, sd>>>(tk, y, d_front_, d_G_,
-                                                                     d_status_);
-                if (side) cudaEventRecord(fev_[1], sd);
-                break;
-            case MF_UPD_NEXT:
-                if (side) cudaStreamWaitEvent(st, fev_[1], 0);
-                if (nb) mf_update64<<<nb, kGThreads, 3 * sizeof(double) * kFTileDoubles, st>>>(
-                    tk, y, d_front_, d_status_);
-                if (side) cudaEventRecord(fev_[0], st);
-                break;
-            case MF_UPDATE:
-                mf_update64<<<nb, kGThreads, 3 * sizeof(double) * kFTileDoubles, st>>>(
-                    tk, y, d_front_, d_status_);
-                break;
-            case MF_INV_T:
-                mf_inv_t64<<<nb, kGThreads, kPairSmem, st>>>(tk, y, d_front_, d_G_, d_status_);
-                break;
-            case MF_INV_X:
-                mf_inv_x64<<<nb, kGThreads, kPairSmem, st>>>(tk, y, d_front_, d_G_, d_status_);
-                break;
-            case MF_WMUL:
-                mf_wmul64<<<nb, kGThreads, kPairSmem, st>>>(tk, y, d_front_, d_G_, d_status_);
-                break;
-        }
-    }
-}
-
-// The launch sequence is fixed by the symbolic analysis, so it is captured
-// once into a CUDA graph and replayed; the shift and the pivot tolerance are
-// read from device memory by the kernels.
 template <> int MultifrontalPlanT<Real>::factorize(const double *d_val, double shift, double pivtol,
                                 cudaStream_t st) {
     if (!d_front_) {
@@ -2254,57 +1265,38 @@ template <> int MultifrontalPlanT<Real>::factorize(const double *d_val, double s
     const double hp[2] = {shift, pivtol};
     cudaMemcpyAsync(d_params_, hp, sizeof hp, cudaMemcpyHostToDevice, st);
     note_h2d(sizeof hp);
-    cudaMemsetAsync(d_status_, 0, sizeof(int), st);
-    if (use_side_ && !fside_) {
-        // the factor graph's second branch (diagonal steps) and its joins;
-        // the branch has the highest priority, so its blocks are scheduled
-        // ahead of the waiting blocks of a large trailing update
-        int prio_lo = 0, prio_hi = 0;
-        cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
-        if (cudaStreamCreateWithPriority(&fside_, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
-            cudaEventCreateWithFlags(&fev_[0], cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&fev_[1], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            return SPEIGS_ERR_INTERNAL;
-        }
-    }
-    bool direct = false;
-    if (!fgraph_ || fgraph_val_ != d_val) {
-        if (fgraph_) { cudaGraphExecDestroy(fgraph_); fgraph_ = nullptr; }
-    }
-    if (!fgraph_ && direct_val_ != d_val) {
-        // the first factorization from these values is launched directly: a
-        // graph pays for its capture only when the plan factors again
-        launch_factor(d_val, st);
-        direct_val_ = d_val;
-        direct = true;
-    } else if (!fgraph_) {
-        cudaGraph_t g = nullptr;
-        if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-            return SPEIGS_ERR_INTERNAL;
-        launch_factor(d_val, st);
-        if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) {
-            cudaGetLastError();
-            return SPEIGS_ERR_INTERNAL;
-        }
-        cudaError_t e = cudaGraphInstantiate(&fgraph_, g, cudaGraphInstantiateFlagUseNodePriority);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { cudaGetLastError(); fgraph_ = nullptr; return SPEIGS_ERR_INTERNAL; }
-        fgraph_val_ = d_val;
-    }
-    if (!direct && cudaGraphLaunch(fgraph_, st) != cudaSuccess) {
+    const size_t nsync = (size_t)nflags_ + ns_ + 3;
+    cudaMemsetAsync(d_fsync_, 0, sizeof(int) * nsync, st);
+    FactorArgs a;
+    a.node = (const FNode *)d_fnode_;
+    a.child = (const FChild *)d_fchild_;
+    a.tasks = (const FTask *)d_ftask_;
+    a.ntasks = nftask_;
+    a.relmap = d_relmap_;
+    a.cbnd = d_cbnd_;
+    a.acolptr = d_acolptr_;
+    a.atpos = d_atpos_;
+    a.asrc = d_asrc_;
+    a.val = d_val;
+    a.params = d_params_;
+    a.F = d_front_;
+    a.G = d_G_;
+    a.flags = d_fsync_;
+    a.upd = d_fsync_ + nflags_;
+    a.queue = a.upd + ns_;
+    a.status = a.queue + 1;
+    a.err = a.queue + 2;
+    mf_factor<<<std::min(factor_grid_, nftask_), kFThreads, sizeof(FShared), st>>>(a);
+    note_launch();
+    int h[2] = {0, 0};
+    cudaMemcpyAsync(h, a.status, sizeof h, cudaMemcpyDeviceToHost, st);
+    note_d2h(sizeof h);
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess || h[1]) {
         cudaGetLastError();
         return SPEIGS_ERR_INTERNAL;
     }
-    long long nk = 0;
-    for (const MfLaunch &L : launches_) nk += L.count > 0;
-    note_launch(nk);
-    int h_status = 0;
-    cudaMemcpyAsync(&h_status, d_status_, sizeof(int), cudaMemcpyDeviceToHost, st);
-    note_d2h(sizeof(int));
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return SPEIGS_ERR_INTERNAL;
-    return h_status ? 1 : 0;
+    return h[0] ? 1 : 0;
 }
 
 template <> void MultifrontalPlanT<Real>::solve(const double *b, double *x, cudaStream_t st,

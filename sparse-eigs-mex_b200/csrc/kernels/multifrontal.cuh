@@ -5,8 +5,8 @@
 // (host/symbolic.h) fixes the supernodes and tree levels; this file owns the
 // device copy of that structure, the tile task lists, and the kernels.
 //
-// Storage.  Every supernode s has a dense front of r x r doubles (column
-// major, rows in the supernode's row-list order) that lives only during the
+// Storage.  Every supernode s has 64 x 64 tiles for its pivot columns, the
+// inverse of their triangle and its update matrix, live only during the
 // factorization, and a persistent r x c panel
 //     G_s = [ inv(L11) ; L21 * inv(L11) ]
 // that replaces the usual [L11 ; L21].  With G, both triangular solves are a
@@ -22,17 +22,6 @@
 #include "../host/symbolic.h"
 
 namespace spx {
-
-constexpr int kTile = 32;
-
-enum MfTaskKind { MF_ASSEMBLE = 0, MF_DIAG, MF_ROWS, MF_UPD_NEXT, MF_UPDATE, MF_INV_T,
-                  MF_INV_X, MF_WMUL, MF_TINY, MF_NKIND };
-
-struct MfLaunch {
-    int     kind;
-    int64_t off;     // first task
-    int64_t count;   // tasks
-};
 
 // Real is the storage type of the fronts and of the panels G: double for
 // the plain FP64 operator, float for the mixed-precision one (FP32 factor,
@@ -86,21 +75,20 @@ public:
     int levels() const { return nlevels_; }
 
 private:
-    void launch_factor(const double *d_val, cudaStream_t st);
     int32_t n_ = 0, ns_ = 0, nlevels_ = 0;
     double flops_ = 0.0;
     int64_t front_total_ = 0, g_total_ = 0, u_total_ = 0, nrows_total_ = 0;
     // device symbolic
-    int32_t *d_perm_ = nullptr, *d_sfirst_ = nullptr, *d_rows_ = nullptr, *d_relmap_ = nullptr;
-    int32_t *d_child_ptr_ = nullptr, *d_child_list_ = nullptr;
-    int64_t *d_rowptr_ = nullptr, *d_frontptr_ = nullptr, *d_gptr_ = nullptr, *d_uptr_ = nullptr;
+    int32_t *d_perm_ = nullptr, *d_rows_ = nullptr, *d_relmap_ = nullptr;
     int32_t *d_acolptr_ = nullptr;   // [n+1] assembly entries per new column
     int32_t *d_atpos_ = nullptr;     // row position within the front
     int32_t *d_asrc_ = nullptr;      // index into the CSR values
-    int32_t *d_cbnd_ = nullptr;      // child bounds per parent 32-row tile
-    int64_t *d_cbnd_ptr_ = nullptr;
-    int4 *d_tasks_ = nullptr;
-    std::vector<MfLaunch> launches_;
+    int32_t *d_cbnd_ = nullptr;      // child bounds per parent 64-row tile
+    // factor: per-supernode metadata, child records, tile task queue, flags
+    void *d_fnode_ = nullptr, *d_fchild_ = nullptr, *d_ftask_ = nullptr;
+    int *d_fsync_ = nullptr;
+    int64_t nflags_ = 0;
+    int nftask_ = 0, factor_grid_ = 0;
     // solve: per-level task offsets (4 lists), tasks, gather lists
     void *d_meta_ = nullptr;         // per-supernode solve metadata
     void *d_stask_ = nullptr;        // solve task queue
@@ -118,8 +106,7 @@ private:
     Real *d_front_ = nullptr;
     Real *d_G_ = nullptr;
     double *d_u_ = nullptr, *d_yf_ = nullptr, *d_x_ = nullptr;
-    int *d_status_ = nullptr;
-    double *d_params_ = nullptr;     // shift, pivot tolerance (read by the graph)
+    double *d_params_ = nullptr;     // shift, pivot tolerance
     // block solve: buffers for rows of up to bw_ doubles (8, 16, 24 or 32)
     // for the right-hand sides, the result, yf, x, the update vectors and
     // the chunk partials; a solve of width NR <= bw_ uses them with stride NR
@@ -129,13 +116,6 @@ private:
            *d_bu_ = nullptr, *d_bfp_ = nullptr, *d_bbp_ = nullptr;
     int bgrid_[4] = {0, 0, 0, 0};          // per width NR = 8 (q + 1): grid, 0 = not set up
     size_t bsmem_[4] = {0, 0, 0, 0};
-    cudaGraphExec_t fgraph_ = nullptr;
-    bool use_side_ = false;                    // some front has >= 2 column blocks
-    cudaStream_t fside_ = nullptr;             // second branch of the factor graph
-    cudaEvent_t fev_[2] = {nullptr, nullptr};  // [0] column kb+1 updated, [1] step kb's panel done
-    const double *fgraph_val_ = nullptr;
-    const double *direct_val_ = nullptr;       // values last factored by direct launches
-    int max_rows_ = 0;
 };
 
 using MultifrontalPlan = MultifrontalPlanT<double>;
@@ -156,8 +136,7 @@ using MultifrontalPlan32 = MultifrontalPlanT<float>;
                                                       const int *, bool);                 \
     template <> void MultifrontalPlanT<R>::release(cudaStream_t);                          \
     template <> int *MultifrontalPlanT<R>::error_word() const;                             \
-    template <> int64_t MultifrontalPlanT<R>::solve_bytes() const;                         \
-    template <> void MultifrontalPlanT<R>::launch_factor(const double *, cudaStream_t);
+    template <> int64_t MultifrontalPlanT<R>::solve_bytes() const;
 SPX_MF_DECLARE(double)
 SPX_MF_DECLARE(float)
 #undef SPX_MF_DECLARE
