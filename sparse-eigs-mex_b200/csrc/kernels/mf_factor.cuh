@@ -40,7 +40,7 @@ constexpr int kFChunk = 16;                    // columns per stage
 enum { FK_DIAG = 0, FK_ROWS, FK_SCHUR, FK_INV, FK_WMUL, FK_SMALL };
 
 struct FNode {          // per-supernode factor metadata (96 bytes)
-    int4 a;             // first column, c, r, ldg
+    int4 a;             // first column, c, r, unused
     int4 b;             // parent, children, first child record, update tiles expected
     longlong2 p;        // pivot tile storage, update tile storage (in Reals)
     longlong2 g;        // panel offset, row-list offset
@@ -122,19 +122,10 @@ SPX_DEV FGeo geo_of(const FNode &nd) {
     return f;
 }
 
-SPX_DEV void dmma(double &d0, double &d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
-}
 SPX_DEV void bar_consumers() { asm volatile("bar.sync 1, %0;" ::"n"(kFConsumers) : "memory"); }
 SPX_DEV void fence_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-SPX_DEV void mbar_init_n(unsigned long long *bar, int n) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
-}
-SPX_DEV void mbar_arrive(unsigned long long *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-// as wait_at_least (bounded), polling without a pause first
+// Bounded wait for *p >= target; gives up (and flags *err) after some
+// seconds, or soon after another wait has given up.
 SPX_DEV void fwait(const int *p, int target, int *err) {
     for (int it = 0; it < 64; it++)
         if (ld_acquire(p) >= target) return;
@@ -541,13 +532,13 @@ SPX_DEV void store_diag(FShared &sh, const Acc &acc, int w, int m0, int n0) {
 
 // X_JJ (w x w lower, zero elsewhere) to the panel, and to tile storage as it
 // is and transposed
-SPX_DEV void write_inverse(const FactorArgs &a, const double *X, int w, Real *Gd, int64_t ldg,
+SPX_DEV void write_inverse(const FactorArgs &a, const double *X, int w, Real *G, int at, int c,
                            Real *L, Real *Xt) {
     const int w4 = round4(w);
     for (int t = threadIdx.x; t < FT * w4; t += kFConsumers) {
         const int i = t & (FT - 1), j = t >> 6;
         const Real lo = (Real)((j < w && i < w && i >= j) ? X[tix<double>(i, j)] : 0.0);
-        if (j < w && i < w && i >= j) Gd[i + (int64_t)j * ldg] = lo;
+        if (j < w && i < w && i >= j) G[gix(at + i, at + j, c)] = lo;
         if (L) {
             L[tix<Real>(i, j)] = lo;
             Xt[tix<Real>(i, j)] = (Real)((i < w && j < w && j >= i) ? X[tix<double>(j, i)] : 0.0);
@@ -561,7 +552,6 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
     const int tid = threadIdx.x, wid = tid >> 5;
     const int m0 = (wid & 1) * 32, n0 = (wid >> 1) * 32;
     Real *Fp = a.F + nd.p.x, *Gp = a.G + nd.g.x;
-    const int64_t ldg = nd.a.w;
     int *fl = a.flags + nd.f.x;
     const int I = tk.I, J = tk.J;
     double *X = reinterpret_cast<double *>(sh.stage);
@@ -576,7 +566,7 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
         if (tk.kind == FK_WMUL) {
             const int ra = f.start(I), ca = f.start(J);
             acc_each(acc, m0, n0, [&](int m, int n, double v) {
-                if (m < h && n < w) Gp[(int64_t)(ra + m) + (int64_t)(ca + n) * ldg] = (Real)v;
+                if (m < h && n < w) Gp[gix(ra + m, ca + n, f.c)] = (Real)v;
             });
             return;
         }
@@ -592,7 +582,7 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
         const int ra = f.start(I), ca = f.start(J), h4 = round4(h);
         acc_each(acc, m0, n0, [&](int m, int n, double v) {
             if (m < h4) Xt[tix<Real>(n, m)] = (Real)(m < h ? -v : 0.0);
-            if (m < h && n < w) Gp[(int64_t)(ra + m) + (int64_t)(ca + n) * ldg] = (Real)-v;
+            if (m < h && n < w) Gp[gix(ra + m, ca + n, f.c)] = (Real)-v;
         });
         publish(fl + f.xflag(J, I));
         return;
@@ -615,7 +605,7 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
             if (i < j || i >= w || j >= w) X[tix<double>(i, j)] = 0.0;
         }
         bar_consumers();
-        write_inverse(a, X, w, Gp, ldg, nullptr, nullptr);
+        write_inverse(a, X, w, Gp, 0, f.c, nullptr, nullptr);
         if (nb > 0) {
             mma_cols(acc, P, X, w4 >> 2, m0, n0, mi, nj);          // L21 = P X^T
             bar_consumers();
@@ -632,7 +622,7 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
             acc_zero(acc);
             mma_cols(acc, P, sh.S, w4 >> 2, m0, n0, mi, nj);
             acc_each(acc, m0, n0, [&](int m, int n, double v) {
-                if (m < nb && n < w) Gp[(int64_t)(w + m) + (int64_t)n * ldg] = (Real)v;
+                if (m < nb && n < w) Gp[gix(w + m, n, f.c)] = (Real)v;
             });
             bar_consumers();
             assemble(a, nd, sh.S, 1, 1, w, nb, w, nb, false);
@@ -684,7 +674,7 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
     store_diag(sh, acc, w, m0, n0);
     bar_consumers();
     chol_inv64(sh.S, X, sh.scratch[0], w, a.params[1], a.status, nd.a.x + ca);
-    write_inverse(a, X, w, Gp + (int64_t)ca + (int64_t)ca * ldg, ldg, Fp + f.ltile(J, J),
+    write_inverse(a, X, w, Gp, ca, f.c, Fp + f.ltile(J, J),
                   Fp + f.xtile(J, J));
     publish(fl + f.lflag(J, J));     // (also orders the ring's reuse by bulk copies)
 }

@@ -23,6 +23,10 @@
 
 namespace spx {
 
+struct SolvePlan {      // one tile queue of the solve
+    int ntasks = 0, fslots = 1, bslots = 1;
+};
+
 // Real is the storage type of the fronts and of the panels G: double for
 // the plain FP64 operator, float for the mixed-precision one (FP32 factor,
 // trailing updates on the TF32 tensor cores with an FP32-accurate 3-term
@@ -89,33 +93,23 @@ private:
     int *d_fsync_ = nullptr;
     int64_t nflags_ = 0;
     int nftask_ = 0, factor_grid_ = 0;
-    // solve: per-level task offsets (4 lists), tasks, gather lists
-    void *d_meta_ = nullptr;         // per-supernode solve metadata
-    void *d_stask_ = nullptr;        // solve task queue
-    int32_t *d_bundle_ = nullptr;
-    int32_t *d_cptr_ = nullptr, *d_cidx_ = nullptr, *d_chunks_ = nullptr;
-    double *d_fpart_ = nullptr, *d_bpart_ = nullptr;
-    int *d_cnt_ = nullptr, *d_sync_ = nullptr;
-    int32_t nfc_ = 0, nbc_ = 0;
-    int ntasks_ = 0;                 // block tasks of the solve queue
-    int nfw_ = 0, nbw_ = 0;          // warp tasks after them: forward, then backward
-    size_t sync_ints_ = 0;
-    int solve_grid_ = 0;
-    size_t solve_smem_ = 0;
+    // solve: tile queues for one right-hand side and for a block, gather
+    // lists; per column count (1, 8, 16, 24, 32) the values that pass between
+    // tasks (two copies), their length and the grid
+    SolvePlan vplan_, bplan_;
+    void *d_vtask_ = nullptr, *d_btask_ = nullptr;
+    int32_t *d_cptr_ = nullptr, *d_cidx_ = nullptr;
+    int *d_sync_ = nullptr;
+    double *d_sval_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    int64_t sstride_[5] = {0, 0, 0, 0, 0};
+    int sgrid_[5] = {0, 0, 0, 0, 0};
+    int solve_setup(int q, cudaStream_t st);
+    int run_solve(int q, const double *B, int64_t ldb, double *X, int64_t ldx, int nr,
+                  cudaStream_t st, const int *skip, bool accumulate);
     // numeric
     Real *d_front_ = nullptr;
     Real *d_G_ = nullptr;
-    double *d_u_ = nullptr, *d_yf_ = nullptr, *d_x_ = nullptr;
     double *d_params_ = nullptr;     // shift, pivot tolerance
-    // block solve: buffers for rows of up to bw_ doubles (8, 16, 24 or 32)
-    // for the right-hand sides, the result, yf, x, the update vectors and
-    // the chunk partials; a solve of width NR <= bw_ uses them with stride NR
-    int bw_ = 0;
-    int32_t fslots_ = 0, bslots_ = 0;
-    double *d_byf_ = nullptr, *d_bx_ = nullptr,
-           *d_bu_ = nullptr, *d_bfp_ = nullptr, *d_bbp_ = nullptr;
-    int bgrid_[4] = {0, 0, 0, 0};          // per width NR = 8 (q + 1): grid, 0 = not set up
-    size_t bsmem_[4] = {0, 0, 0, 0};
 };
 
 using MultifrontalPlan = MultifrontalPlanT<double>;
@@ -134,6 +128,10 @@ using MultifrontalPlan32 = MultifrontalPlanT<float>;
     template <> int MultifrontalPlanT<R>::solve_block(const double *, int64_t, double *,   \
                                                       int64_t, int, cudaStream_t,         \
                                                       const int *, bool);                 \
+    template <> int MultifrontalPlanT<R>::solve_setup(int, cudaStream_t);                  \
+    template <> int MultifrontalPlanT<R>::run_solve(int, const double *, int64_t,          \
+                                                    double *, int64_t, int, cudaStream_t,  \
+                                                    const int *, bool);                    \
     template <> void MultifrontalPlanT<R>::release(cudaStream_t);                          \
     template <> int *MultifrontalPlanT<R>::error_word() const;                             \
     template <> int64_t MultifrontalPlanT<R>::solve_bytes() const;
