@@ -1365,8 +1365,12 @@ static double wall() {
 struct speigs_plan_s {
     spx::Stream stream;
     spx::HostCSR A;                  // full symmetric CSR (host copy of the pattern)
-    std::vector<int64_t> csc2csr;    // per CSC entry: CSR position(s) it feeds, or -1
-    int64_t csc_nnz = 0;
+    // set_values: the CSC entry each CSR value comes from, and the caller's
+    // values, both on the device; map_state 0: not made yet, 1: in use, -1:
+    // the columns are not strictly sorted, the host rebuilds the CSR
+    int32_t *d_map = nullptr;
+    double *d_ax = nullptr;
+    int map_state = 0;
     std::vector<int64_t> Ap_copy;    // CSC column pointers given at creation
     std::vector<int64_t> Ai_copy;
     speigs_which which = SPEIGS_SM;
@@ -2492,8 +2496,51 @@ int speigs_plan_create_ex(speigs_int n, const speigs_int *Ap, const speigs_int *
     return SPEIGS_OK;
 }
 
+// The device path of speigs_plan_set_values.  Returns 0, a negative code, or 1
+// when the host has to rebuild the CSR.
+static int plan_set_values_device(speigs_plan p, const double *Ax) {
+    using namespace spx;
+    cudaStream_t st = p->stream.s;
+    const int n = p->A.n;
+    const int64_t nnz = p->A.nnz(), cnnz = (int64_t)p->Ai_copy.size();
+    if (p->map_state < 0 || cnnz > INT32_MAX) return 1;
+    Arena ar(st);
+    if (p->map_state == 0) {
+        int rc = plan_alloc(p, (void **)&p->d_map, sizeof(int32_t) * nnz);
+        rc = rc ? rc : plan_alloc(p, (void **)&p->d_ax, sizeof(double) * cnnz);
+        if (rc) return rc;
+        int64_t *dAp = ar.alloc<int64_t>(n + 1), *dAi = ar.alloc<int64_t>(cnnz);
+        int *bad = ar.alloc<int>(1);
+        if (ar.failed) return SPEIGS_ERR_MEM;
+        copy_async(dAp, p->Ap_copy.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
+        copy_async(dAi, p->Ai_copy.data(), sizeof(int64_t) * cnnz, cudaMemcpyHostToDevice, st);
+        cudaMemsetAsync(bad, 0, sizeof(int), st);
+        launch_csc_map(n, dAp, dAi, p->d_rp, p->d_ci, p->d_map, bad, st);
+        int h_bad = 0;
+        copy_async(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaError_t e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return cuda_fail(e, "value map");
+        p->map_state = h_bad ? -1 : 1;
+        if (h_bad) return 1;
+    }
+    unsigned long long *bits = ar.alloc<unsigned long long>(1);
+    if (ar.failed) return SPEIGS_ERR_MEM;
+    p->factored = false;
+    cudaMemsetAsync(bits, 0, sizeof *bits, st);
+    copy_async(p->d_ax, Ax, sizeof(double) * cnnz, cudaMemcpyHostToDevice, st);
+    launch_csc_values(n, p->d_rp, p->d_map, p->d_ax, p->d_va, bits, st);
+    double anorm = 0.0;
+    copy_async(&anorm, bits, sizeof anorm, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(e, "new values");
+    p->anorm = anorm > 0 ? anorm : 1.0;
+    return 0;
+}
+
 int speigs_plan_set_values(speigs_plan p, const double *Ax) {
     if (!p || !Ax) return SPEIGS_ERR_ARG;
+    const int dev_rc = plan_set_values_device(p, Ax);
+    if (dev_rc <= 0) return dev_rc;
     const int64_t n = p->A.n;
     HostCSR B;
     int rc = spx::build_full_csr(n, p->Ap_copy.data(), p->Ai_copy.data(), Ax, &B);

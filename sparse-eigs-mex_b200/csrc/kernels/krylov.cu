@@ -880,4 +880,69 @@ Counters &counters() {
     static Counters c;
     return c;
 }
+// ------------------------------------------------------- new values ------
+// Bound by the copy of the caller's values to the device; the host rebuilt the
+// whole CSR for this before (7.8 ms at 48^3, 760,000 entries; 0.9 ms now).
+__global__ void csc_map_kernel(int n, const int64_t *__restrict__ Ap, const int64_t *__restrict__ Ai,
+                               const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                               int32_t *__restrict__ map, int *bad) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    // the place of column `col` in row `row`, or -1
+    auto find = [&](int row, int col) {
+        int lo = rp[row], hi = rp[row + 1];
+        const int end = hi;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (ci[mid] < col) lo = mid + 1; else hi = mid;
+        }
+        return lo < end && ci[lo] == col ? lo : -1;
+    };
+    int64_t last = -1;
+    bool ok = true;
+    for (int64_t q = Ap[c]; q < Ap[c + 1]; q++) {
+        const int64_t r = Ai[q];
+        if (r <= last || r >= n) { ok = false; break; }
+        last = r;
+        if (r > c) continue;
+        const int d = find((int)r, c), e = r < c ? find(c, (int)r) : d;
+        if (d < 0 || e < 0) { ok = false; break; }
+        map[d] = (int32_t)q;
+        map[e] = (int32_t)q;
+    }
+    if (!ok) *bad = 1;
+}
+void launch_csc_map(int n, const int64_t *Ap, const int64_t *Ai, const int32_t *rp,
+                    const int32_t *ci, int32_t *map, int *bad, cudaStream_t st) {
+    csc_map_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, Ap, Ai, rp, ci, map, bad);
+    note_launch();
+}
+
+__global__ void csc_values_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ map,
+                                  const double *__restrict__ ax, double *__restrict__ va,
+                                  unsigned long long *norm_bits) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    double s = 0.0;
+    if (r < n)
+        for (int q = rp[r]; q < rp[r + 1]; q++) {
+            const double v = ax[map[q]];
+            va[q] = v;
+            s += fabs(v);
+        }
+    // the maximum over rows, NaN rows left out; sums are not negative, so
+    // their bits are ordered as they are
+    unsigned long long b = s > 0.0 ? (unsigned long long)__double_as_longlong(s) : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
+        b = t > b ? t : b;
+    }
+    if ((threadIdx.x & 31) == 0 && b) atomicMax(norm_bits, b);
+}
+void launch_csc_values(int n, const int32_t *rp, const int32_t *map, const double *ax, double *va,
+                       unsigned long long *norm_bits, cudaStream_t st) {
+    csc_values_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, rp, map, ax, va, norm_bits);
+    note_launch();
+}
+
 }  // namespace spx

@@ -111,4 +111,16 @@ void launch_axpby(int64_t n, double a, const double *x, double b, double *y, cud
 void launch_copy(int64_t n, const double *src, double *dst, cudaStream_t st);
 void launch_fill(int64_t n, double v, double *dst, cudaStream_t st);
 
+// New values for a plan's matrix from its caller's CSC, on the device.
+// launch_csc_map: map[q] = the CSC entry whose value CSR position q holds (the
+// CSR of the upper triangle's symmetric matrix, columns ascending); raises
+// *bad when a column's row indices are not strictly increasing or an entry is
+// not found, and the map is then not to be used.  launch_csc_values: the CSR
+// values through the map, and in *norm_bits the bits of ||A||_1 (zero on
+// entry), each row summed in order.
+void launch_csc_map(int n, const int64_t *Ap, const int64_t *Ai, const int32_t *rp,
+                    const int32_t *ci, int32_t *map, int *bad, cudaStream_t st);
+void launch_csc_values(int n, const int32_t *rp, const int32_t *map, const double *ax, double *va,
+                       unsigned long long *norm_bits, cudaStream_t st);
+
 }  // namespace spx
