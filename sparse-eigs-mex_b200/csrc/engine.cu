@@ -14,6 +14,7 @@
 #include "kernels/multifrontal.cuh"
 #include "kernels/block_krylov.cuh"
 #include "kernels/dense_lu.cuh"
+#include "kernels/dense_eig.cuh"
 #include "kernels/seg_lanczos.cuh"
 #include "counters.h"
 #include "host/syev_host.h"
@@ -2383,6 +2384,75 @@ __global__ void densify_kernel(int n, const int32_t *rp, const int32_t *ci, cons
             D[(size_t)r + (size_t)ci[q] * n] = va[q];
 }
 
+// A few eigenpairs by reduction to tridiagonal form (dense_eig.cuh).  Returns 0
+// with lambda (sorted by |lambda|) and V, a negative code, or 1 when the
+// Jacobi solver has to do it: an entry out of the range whose squares are
+// safe, or pairs that miss the check of their residuals.
+static int dense_few_pairs(int n, const double *D, int k, speigs_which which, double amax,
+                           double *lambda, double *V, Arena &ar, cudaStream_t st) {
+    if (n < kDenseEigMin || n > kDenseEigMax || k > kDenseEigMaxK || !(amax < 1e100) ||
+        (amax < 1e-100 && amax != 0.0))
+        return 1;
+    double *Q = ar.alloc<double>((size_t)n * n);
+    double *work = dense_tridiag_work(n) ? ar.alloc<double>((size_t)n * n) : nullptr;
+    double *td = ar.alloc<double>(3 * (size_t)n + 4 * (size_t)k);     // d, e, beta, candidates, lambda, residuals
+    double *te = td + n, *tb = te + n, *tv = tb + n, *tl = tv + 2 * k, *tr = tl + k;
+    int *ti = ar.alloc<int>(2 * (size_t)k);
+    double *Z = ar.alloc<double>((size_t)n * k);
+    if (ar.failed) return SPEIGS_ERR_MEM;
+    if (launch_dense_tridiag(n, D, Q, tb, td, te, work, st) != cudaSuccess) {
+        cudaGetLastError();          // a cluster of that size is not to be had
+        return 1;
+    }
+    launch_tri_bisect(n, td, te, k, which == SPEIGS_SM, tv, ti, st);
+    std::vector<double> h(2 * (size_t)n + 2 * (size_t)k);
+    std::vector<int> hi(2 * (size_t)k);
+    copy_async(h.data(), td, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, st);
+    copy_async(h.data() + 2 * n, tv, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, st);
+    copy_async(hi.data(), ti, sizeof(int) * 2 * k, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(e, "dense path");
+    // the k wanted of the candidates (ascending, each once), by |theta|, ties
+    // in ascending order
+    std::vector<double> cand;
+    for (int w = 0; w < 2 * k; w++)
+        if (hi[w] >= 0 && (w == 0 || hi[w] != hi[w - 1])) cand.push_back(h[2 * n + w]);
+    if ((int)cand.size() < k) return 1;
+    for (size_t c = 1; c < cand.size(); c++) cand[c] = std::max(cand[c], cand[c - 1]);
+    auto by_magnitude = [&](const std::vector<double> &v) {
+        std::vector<int> o(v.size());
+        for (size_t i = 0; i < o.size(); i++) o[i] = (int)i;
+        std::stable_sort(o.begin(), o.end(), [&](int a, int b) {
+            return which == SPEIGS_SM ? fabs(v[a]) < fabs(v[b]) : fabs(v[a]) > fabs(v[b]);
+        });
+        return o;
+    };
+    std::vector<int> pick = by_magnitude(cand);
+    pick.resize(k);
+    std::sort(pick.begin(), pick.end());
+    std::vector<double> lam(k), zh((size_t)n * k);
+    for (int t = 0; t < k; t++) lam[t] = cand[pick[t]];
+    if (tri_vectors_host(n, h.data(), h.data() + n, k, lam.data(), zh.data()) != 0) return 1;
+    copy_async(Z, zh.data(), sizeof(double) * (size_t)n * k, cudaMemcpyHostToDevice, st);
+    launch_apply_reflectors(n, Q, tb, Z, k, st);
+    launch_rayleigh_dd(n, D, Z, k, tl, tr, st);
+    std::vector<double> q(2 * (size_t)k);
+    copy_async(q.data(), tl, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, st);
+    e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(e, "dense path");
+    for (int t = 0; t < k; t++)
+        if (!(sqrt(q[k + t]) <= 1e-13 * n * amax)) return 1;
+    q.resize(k);
+    const std::vector<int> o = by_magnitude(q);
+    for (int t = 0; t < k; t++) {
+        lambda[t] = q[o[t]];
+        if (V) copy_async(V + (size_t)t * n, Z + (size_t)o[t] * n, sizeof(double) * n,
+                          cudaMemcpyDeviceToHost, st);
+    }
+    e = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? 0 : cuda_fail(e, "dense path copy");
+}
+
 int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *lambda,
                       double *V, double *resid, speigs_info *info) {
     g_err[0] = 0;
@@ -2401,12 +2471,6 @@ int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *l
         int32_t *d_ci = ar.alloc<int32_t>(nnz);
         double *d_va = ar.alloc<double>(nnz);
         double *D = ar.alloc<double>((size_t)n * n);
-        double *th = ar.alloc<double>(n);
-        double *S = ar.alloc<double>((size_t)n * n);
-        int *od = ar.alloc<int>(n);
-        int *stt = ar.alloc<int>(2);
-        const int me = (n + 1) & ~1;
-        double *work = (n > syev_small_smem_limit()) ? ar.alloc<double>((size_t)2 * me * me) : nullptr;
         if (ar.failed) return SPEIGS_ERR_MEM;
         copy_async(d_rp, rp32.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, st);
         copy_async(d_ci, A.col, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, st);
@@ -2414,6 +2478,27 @@ int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *l
         cudaMemsetAsync(D, 0, sizeof(double) * n * n, st);
         densify_kernel<<<std::min(n, 4096), 32, 0, st>>>(n, d_rp, d_ci, d_va, D);
         note_launch();
+        double amax = 0.0;
+        for (int64_t q = 0; q < nnz; q++) {
+            if (!std::isfinite(A.val[q])) { amax = NAN; break; }
+            amax = std::max(amax, fabs(A.val[q]));
+        }
+        const int few = dense_few_pairs(n, D, (int)k, which, amax, lambda, V, ar, st);
+        if (few <= 0) {
+            if (few < 0) return few;
+            for (int64_t t = 0; t < k && resid; t++) resid[t] = 0.0;
+            info->nconv = k;
+            info->flag = 0;
+            info->path = SPEIGS_PATH_DENSE;
+            return SPEIGS_OK;
+        }
+        double *th = ar.alloc<double>(n);
+        double *S = ar.alloc<double>((size_t)n * n);
+        int *od = ar.alloc<int>(n);
+        int *stt = ar.alloc<int>(2);
+        const int me = (n + 1) & ~1;
+        double *work = (n > syev_small_smem_limit()) ? ar.alloc<double>((size_t)2 * me * me) : nullptr;
+        if (ar.failed) return SPEIGS_ERR_MEM;
         launch_syev_small(n, D, n, th, S, od, work, stt, st);
         int hst[2] = {0, 0};
         copy_async(theta.data(), th, sizeof(double) * n, cudaMemcpyDeviceToHost, st);

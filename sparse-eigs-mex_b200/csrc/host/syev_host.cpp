@@ -243,8 +243,7 @@ void apply_q(int n, const std::vector<double> &V, const std::vector<double> &bet
 struct TriLU {
     std::vector<double> u0, u1, u2, l;
     std::vector<char> swp;
-    void factor(int n, const std::vector<double> &d, const std::vector<double> &e, double sigma,
-                double tiny) {
+    void factor(int n, const double *d, const double *e, double sigma, double tiny) {
         u0.assign(n, 0.0); u1.assign(n, 0.0); u2.assign(n, 0.0); l.assign(n, 0.0);
         swp.assign(n, 0);
         // pending row i: x0 (column i), x1 (i+1), x2 (i+2)
@@ -281,6 +280,49 @@ struct TriLU {
 
 }  // namespace
 
+int tri_vectors_host(int m, const double *d0, const double *e0, int nvec, const double *lam,
+                     double *Zw) {
+    // a cluster is a run whose neighbours lie within 1e-3 ||T||_inf, and each
+    // vector is kept orthogonal to those computed before it in its cluster
+    double tnorm = 0.0;
+    for (int i = 0; i < m; i++)
+        tnorm = std::max(tnorm, std::fabs(d0[i]) + (i > 0 ? std::fabs(e0[i - 1]) : 0.0) +
+                                    (i + 1 < m ? std::fabs(e0[i]) : 0.0));
+    if (tnorm == 0.0) tnorm = 1.0;
+    const double tiny = DBL_EPSILON * tnorm, ortol = 1e-3 * tnorm;
+    TriLU lu;
+    std::vector<double> z(m);
+    int clus = 0;                                   // first vector of the current cluster
+    uint64_t rs = 0x9E3779B97F4A7C15ULL;
+    for (int w = 0; w < nvec; w++) {
+        if (w == 0 || lam[w] - lam[w - 1] > ortol) clus = w;
+        lu.factor(m, d0, e0, lam[w], tiny);
+        for (int i = 0; i < m; i++) {                // start: uniform in [-1, 1] (xorshift64*)
+            rs ^= rs >> 12; rs ^= rs << 25; rs ^= rs >> 27;
+            z[i] = 2.0 * (double)((rs * 0x2545F4914F6CDD1DULL) >> 11) / 9007199254740992.0 - 1.0;
+        }
+        for (int it = 0; it < 3; it++) {
+            double mx = 0.0;
+            for (int i = 0; i < m; i++) mx = std::max(mx, std::fabs(z[i]));
+            for (int i = 0; i < m; i++) z[i] /= mx;
+            lu.solve(m, z.data());
+            for (int c = clus; c < w; c++) {
+                const double *q = Zw + (size_t)c * m;
+                double dot = 0.0;
+                for (int i = 0; i < m; i++) dot += q[i] * z[i];
+                for (int i = 0; i < m; i++) z[i] -= dot * q[i];
+            }
+        }
+        double nrm = 0.0;
+        for (int i = 0; i < m; i++) nrm += z[i] * z[i];
+        nrm = std::sqrt(nrm);
+        if (!(nrm > 0.0) || !std::isfinite(nrm)) return -1;
+        for (int i = 0; i < m; i++) z[i] /= nrm;
+        std::memcpy(Zw + (size_t)w * m, z.data(), sizeof(double) * m);
+    }
+    return 0;
+}
+
 int syev_host_select(int m, const double *H, int ldh, int nvec, double *theta, double *S,
                      int *ord) {
     if (m <= 0) return 0;
@@ -305,48 +347,11 @@ int syev_host_select(int m, const double *H, int ldh, int nvec, double *theta, d
                      [&](int a, int b) { return std::fabs(theta[a]) > std::fabs(theta[b]); });
     std::memset(S, 0, sizeof(double) * (size_t)m * m);
     if (nvec <= 0) return steps;
-    // the wanted eigenvalues in ascending order; a cluster is a run whose
-    // neighbours lie within 1e-3 ||T||_inf, and each vector is kept
-    // orthogonal to those computed before it in its cluster
-    std::vector<int> want(ord, ord + nvec);
+    std::vector<int> want(ord, ord + nvec);         // the wanted eigenvalues, ascending
     std::sort(want.begin(), want.end());
-    double tnorm = 0.0;
-    for (int i = 0; i < m; i++)
-        tnorm = std::max(tnorm, std::fabs(d0[i]) + (i > 0 ? std::fabs(e0[i - 1]) : 0.0) +
-                                    (i + 1 < m ? std::fabs(e0[i]) : 0.0));
-    if (tnorm == 0.0) tnorm = 1.0;
-    const double tiny = DBL_EPSILON * tnorm, ortol = 1e-3 * tnorm;
-    TriLU lu;
-    std::vector<double> z(m), Zw((size_t)m * want.size());
-    std::vector<std::vector<double>> clus;          // eigenvectors of T in the current cluster
-    uint64_t rs = 0x9E3779B97F4A7C15ULL;
-    for (size_t w = 0; w < want.size(); w++) {
-        const int j = want[w];
-        if (w == 0 || theta[j] - theta[want[w - 1]] > ortol) clus.clear();
-        lu.factor(m, d0, e0, theta[j], tiny);
-        for (int i = 0; i < m; i++) {                // start: uniform in [-1, 1] (xorshift64*)
-            rs ^= rs >> 12; rs ^= rs << 25; rs ^= rs >> 27;
-            z[i] = 2.0 * (double)((rs * 0x2545F4914F6CDD1DULL) >> 11) / 9007199254740992.0 - 1.0;
-        }
-        for (int it = 0; it < 3; it++) {
-            double mx = 0.0;
-            for (int i = 0; i < m; i++) mx = std::max(mx, std::fabs(z[i]));
-            for (int i = 0; i < m; i++) z[i] /= mx;
-            lu.solve(m, z.data());
-            for (const auto &q : clus) {
-                double dot = 0.0;
-                for (int i = 0; i < m; i++) dot += q[i] * z[i];
-                for (int i = 0; i < m; i++) z[i] -= dot * q[i];
-            }
-        }
-        double nrm = 0.0;
-        for (int i = 0; i < m; i++) nrm += z[i] * z[i];
-        nrm = std::sqrt(nrm);
-        if (!(nrm > 0.0) || !std::isfinite(nrm)) return -1;
-        for (int i = 0; i < m; i++) z[i] /= nrm;
-        clus.push_back(z);
-        std::memcpy(Zw.data() + w * m, z.data(), sizeof(double) * m);
-    }
+    std::vector<double> wl(want.size()), Zw((size_t)m * want.size());
+    for (size_t w = 0; w < want.size(); w++) wl[w] = theta[want[w]];
+    if (tri_vectors_host(m, d0.data(), e0.data(), (int)want.size(), wl.data(), Zw.data()) != 0) return -1;
     apply_q(m, V, beta, Zw.data(), (int)want.size());
     for (size_t w = 0; w < want.size(); w++)
         std::memcpy(S + (size_t)want[w] * m, Zw.data() + w * m, sizeof(double) * m);

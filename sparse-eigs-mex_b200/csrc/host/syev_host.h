@@ -23,4 +23,12 @@ int syev_host(int m, const double *H, int ldh, double *theta, double *S, int *or
 int syev_host_select(int m, const double *H, int ldh, int nvec, double *theta, double *S,
                      int *ord);
 
+// Unit eigenvectors of the symmetric tridiagonal (d[n], e[n-1]) for nvec of
+// its eigenvalues lam (ascending): inverse iteration, each vector kept
+// orthogonal to the earlier ones of its cluster (neighbours within
+// 1e-3 ||T||_inf).  Z: n x nvec, ld n.  Returns 0, or -1 when a vector could
+// not be normalised.
+int tri_vectors_host(int n, const double *d, const double *e, int nvec, const double *lam,
+                     double *Z);
+
 }  // namespace spx
