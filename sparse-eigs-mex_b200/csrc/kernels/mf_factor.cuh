@@ -27,11 +27,14 @@
 // the FP64 tensor cores, each a 32 x 32 quarter of the tile in registers.
 //
 // What bounds it: at the top of the tree the chain of diagonal tiles of the
-// large separators (about 15 us a column block; a launch per step took 55),
-// elsewhere the FP64 pipe.  Measured on 3-D grids, against one launch per
-// column-block step (graph of 590 launches at 48^3) on the narrower
-// supernodes of before: 20^3 2.0 -> 0.66 ms, 33x35x37 4.67 -> 1.94, 48^3
-// 9.84 -> 4.73, 64^3 28.8 -> 15.7.
+// large separators (about 30 us a column block: 11 us for the 64 x 64
+// Cholesky and inverse, two tile products and three hand-overs of about 2 us;
+// a launch per step took 55), elsewhere the tiles' latencies -- 5 us of
+// assembly and 3 us of stores around 2.2 us a product, two tiles an SM -- and
+// then the FP64 pipe (1.4 of 4.4 ms at 48^3, 7.6 of 15.7 at 64^3).  Measured
+// on 3-D grids, against one launch per column-block step (a graph of 590
+// launches at 48^3) on the narrower supernodes of before: 20^3 2.0 -> 0.63 ms,
+// 33x35x37 4.67 -> 1.76, 48^3 9.84 -> 4.45, 64^3 28.8 -> 15.7.
 constexpr int FT = 64;
 constexpr int kFConsumers = 128;
 constexpr int kFThreads = kFConsumers + 32;
@@ -61,7 +64,8 @@ struct FactorArgs {
     const FChild *child;
     const FTask *tasks;
     int ntasks;
-    const int32_t *relmap, *cbnd, *acolptr, *atpos, *asrc;
+    const int32_t *relmap, *cbnd, *acolptr, *atpos, *acolj, *asrc;
+    int dup;                     // some entry of A is stored more than once
     const double *val;
     const double *params;        // shift, pivot tolerance
     Real *F, *G;
@@ -233,11 +237,12 @@ SPX_DEV void assemble(const FactorArgs &a, const FNode &nd, double *S, int I, in
             for (int v = 0; v < 2; v++) {
                 unsigned mine = __ballot_sync(full, rj[v] >= 0 && (rj[v] & 3) == wid);
                 while (mine) {
-                    // up to four columns at a time, their loads in flight together
-                    int jc[4], tj[4];
-                    double x0[4], x1[4];
+                    // up to eight columns at a time, their loads in flight together
+                    constexpr int U = 8;
+                    int jc[U], tj[U];
+                    double x0[U], x1[U];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
+                    for (int e = 0; e < U; e++) {
                         jc[e] = mine ? __ffs(mine) - 1 : -1;
                         mine &= mine - 1;
                         tj[e] = __shfl_sync(full, rj[v], jc[e] < 0 ? 0 : jc[e]);
@@ -256,7 +261,7 @@ SPX_DEV void assemble(const FactorArgs &a, const FNode &nd, double *S, int I, in
                         }
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
+                    for (int e = 0; e < U; e++) {
                         if (jc[e] >= 0) {
                             if (ri[0] >= 0) S[tix<double>(ri[0], tj[e])] += x0[e];
                             if (ri[1] >= 0) S[tix<double>(ri[1], tj[e])] += x1[e];
@@ -269,13 +274,22 @@ SPX_DEV void assemble(const FactorArgs &a, const FNode &nd, double *S, int I, in
         }
     }
     if (pivots) {
+        const int col0 = nd.a.x + ca;
+        const int e0 = a.acolptr[col0], e1 = a.acolptr[col0 + w];
         bar_consumers();
-        if (tid < w) {
-            const int col = nd.a.x + ca + tid;
-            const int e1 = a.acolptr[col + 1];
-            for (int e = a.acolptr[col]; e < e1; e++) {
-                const int tp = a.atpos[e] - ra;
-                if (tp >= 0 && tp < h) S[tix<double>(tp, tid)] += a.val[a.asrc[e]];
+        if (!a.dup) {
+            // the columns' entries are one range: a thread an entry
+            for (int e = e0 + tid; e < e1; e += kFConsumers) {
+                const int i = a.atpos[e] - ra;
+                if (i >= 0 && i < h) S[tix<double>(i, a.acolj[e] - col0)] += a.val[a.asrc[e]];
+            }
+            bar_consumers();
+            if (I == J && tid < w) S[tix<double>(tid, tid)] += a.params[0];
+        } else if (tid < w) {
+            // repeated entries are added in their order: a thread a column
+            for (int e = a.acolptr[col0 + tid]; e < a.acolptr[col0 + tid + 1]; e++) {
+                const int i = a.atpos[e] - ra;
+                if (i >= 0 && i < h) S[tix<double>(i, tid)] += a.val[a.asrc[e]];
             }
             if (I == J) S[tix<double>(tid, tid)] += a.params[0];
         }
@@ -283,31 +297,51 @@ SPX_DEV void assemble(const FactorArgs &a, const FNode &nd, double *S, int I, in
     bar_consumers();
 }
 
-// 8 x 8 block products on one warp: fragment loads from tiles in the S layout
-SPX_DEV double fragA(const double *M, int i0, int k0, int ks) {
-    const int lane = threadIdx.x & 31;
-    return M[tix<double>(i0 + (lane >> 2), k0 + 4 * ks + (lane & 3))];
-}
-// B^T operand: element (n, k)
-SPX_DEV double fragBt(const double *M, int n0, int k0, int ks) { return fragA(M, n0, k0, ks); }
-// B operand: element (k, n)
-SPX_DEV double fragB(const double *M, int k0, int n0, int ks) {
-    const int lane = threadIdx.x & 31;
-    return M[tix<double>(k0 + 4 * ks + (lane & 3), n0 + (lane >> 2))];
-}
+// Places of an 8 x 8 block's elements in a tile of the S layout, as a lane's
+// constants plus one XOR and one add a block (the blocks start at multiples of
+// 8, so the layout's XOR splits into its bit 3 and the bits below):
+//   nn: element (row0 + lane / 4, col0 + 4 ks + lane % 4), ks = 0, 1
+//   tn: element (row0 + 4 ks + lane % 4, col0 + lane / 4)
+//   cc: element (row0 + lane / 4, col0 + 2 (lane % 4) + e), e = 0, 1
+struct Blk8 {
+    int a0, ax, b0[2], bx, c0[2], cx[2];
+    SPX_DEV Blk8() {
+        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+        a0 = t * FT + (g ^ ((t << 2) & 4));
+        ax = (t << 2) & 8;
+        const int c = (g & 3) << 2;
+        bx = c & 8;
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++) b0[ks] = g * FT + ((4 * ks) ^ (c & 4)) + t;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int q = ((2 * t + e) & 3) << 2;
+            c0[e] = (2 * t + e) * FT + (g ^ (q & 4));
+            cx[e] = q & 8;
+        }
+    }
+    SPX_DEV int nn(int row0, int col0, int ks) const { return a0 + (row0 ^ ax) + (col0 + 4 * ks) * FT; }
+    SPX_DEV int tn(int row0, int col0, int ks) const { return b0[ks] + (row0 ^ bx) + col0 * FT; }
+    SPX_DEV int cc(int row0, int col0, int e) const { return c0[e] + (row0 ^ cx[e]) + col0 * FT; }
+};
 
-// Cholesky factor and inverse of one 8 x 8 block, by a whole warp: every
-// lane factors the block in its own registers (no exchanges on the chain of
-// pivots), then computes column lane % 8 of the inverse; lanes 0..7 write
-// X_pp.  A pivot <= pivtol records its column and is replaced by 1.
-__device__ __noinline__ void chol8(const double *D, double *X, int o, double pivtol, int *status,
+// Cholesky factor and inverse of one 8 x 8 block, by a whole warp: every lane
+// factors the block in its own registers (no exchanges on the chain of
+// pivots) and carries column lane % 8 of the identity along, which leaves
+// that column of the inverse; lanes 0..7 write X_pp.  A pivot <= pivtol
+// records its column and is replaced by 1.
+SPX_DEV void chol8(const double *D, double *X, int o, double pivtol, int *status,
                                    int colbase, int w) {
-    const int lane = threadIdx.x & 31;
-    double l[8][8], rl[8];
+    const int lane = threadIdx.x & 31, c = lane & 7;
+    double l[8][8], x[8];
+    // the block's columns with bit 3 of the layout's XOR clear and set
+    const double *p0 = D + o * FT + o, *p8 = D + o * FT + (o ^ 8);
 #pragma unroll
     for (int j = 0; j < 8; j++)
 #pragma unroll
-        for (int i = j; i < 8; i++) l[i][j] = D[tix<double>(o + i, o + j)];
+        for (int i = j; i < 8; i++) l[i][j] = ((j & 2) ? p8 : p0)[j * FT + (i ^ ((j & 1) << 2))];
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i] = (i == c) ? 1.0 : 0.0;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
         double d = l[j][j];
@@ -315,26 +349,22 @@ __device__ __noinline__ void chol8(const double *D, double *X, int o, double piv
             if (lane == 0 && o + j < w) atomicCAS(status, 0, colbase + o + j + 1);
             d = 1.0;
         }
-        rl[j] = rsqrt(d);
+        const double r = rsqrt(d);
 #pragma unroll
-        for (int i = j + 1; i < 8; i++) l[i][j] *= rl[j];
+        for (int i = j + 1; i < 8; i++) l[i][j] *= r;
 #pragma unroll
         for (int k = j + 1; k < 8; k++)
 #pragma unroll
             for (int i = k; i < 8; i++) l[i][k] -= l[i][j] * l[k][j];
+        x[j] *= r;
+#pragma unroll
+        for (int i = j + 1; i < 8; i++) x[i] -= l[i][j] * x[j];
     }
-    const int c = lane & 7;
-    double x[8];
+    if (lane < 8) {
+        double *q = X + (o + c) * FT + (o ^ ((c & 2) << 2));
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        double s = (i == c) ? 1.0 : 0.0;
-#pragma unroll
-        for (int k = 0; k < i; k++) s -= l[i][k] * x[k];
-        x[i] = s * rl[i];            // zero above the diagonal: every term is
+        for (int i = 0; i < 8; i++) q[i ^ ((c & 1) << 2)] = x[i];
     }
-    if (lane < 8)
-#pragma unroll
-        for (int i = 0; i < 8; i++) X[tix<double>(o + i, o + c)] = x[i];
     __syncwarp();
 }
 
@@ -344,46 +374,30 @@ __device__ __noinline__ void chol8(const double *D, double *X, int o, double piv
 // off-diagonal blocks L_ip are left transposed in place: block (i, p) of L at
 // block (p, i) of D.  Per 8 pivots: warp 0 runs the chain (block p+1's row,
 // update, factor), warps 1-3 the rest of the panel, the trailing update and
-// row p of the inverse beside it.
+// row p of the inverse beside it, each in groups of independent blocks: the
+// blocks' latencies, not their products, are what they cost.  21,300 cycles for
+// a full tile (26,000 with one block at a time); the chain alone, a factored
+// 8 x 8 block every 1,970 cycles, is 15,800 of them.
 SPX_DEV void chol_inv64(double *D, double *X, double *scr, int w, double pivtol, int *status,
                         int colbase) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3, nb = (w + 7) >> 3;
-    // L_ip = A_ip X_pp^T to dst(i', k') = L(i', k') in the S layout at (di, dk)
-    auto panel = [&](int i, int p, double &d0, double &d1) {
-        d0 = d1 = 0.0;
+    const Blk8 at;
+#pragma unroll 1
+    for (int p = -1; p < nb; p++) {                      // p = -1: the first block alone
+        double xp[2] = {0.0, 0.0};
+        if (p >= 0)
 #pragma unroll
-        for (int ks = 0; ks < 2; ks++)
-            dmma(d0, d1, fragA(D, 8 * i, 8 * p, ks), fragBt(X, 8 * p, 8 * p, ks));
-    };
-    // row p of the inverse, block (p, j): X_pj = -X_pp sum_k L_pk X_kj
-    auto xrow = [&](int p, int j) {
-        double y0 = 0.0, y1 = 0.0;
-        for (int k = j; k < p; k++)
+            for (int ks = 0; ks < 2; ks++) xp[ks] = X[at.nn(8 * p, 8 * p, ks)];
+        if (wid == 0 && p + 1 < nb) {
+            const int i = p + 1;
+            if (p >= 0) {
+                const int c0 = at.cc(8 * i, 8 * i, 0), c1 = at.cc(8 * i, 8 * i, 1);
+                const double e0 = D[c0], e1 = D[c1];
+                double d0 = 0.0, d1 = 0.0;                   // L_ip = A_ip X_pp^T
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++)       // L_pk(m, q) is at D(8k + q, 8p + m)
-                dmma(y0, y1, D[tix<double>(8 * k + 4 * ks + t, 8 * p + g)], fragB(X, 8 * k, 8 * j, ks));
-        double r0 = 0.0, r1 = 0.0;
-#pragma unroll
-        for (int ks = 0; ks < 2; ks++) {
-            // accumulator (row g, columns 2t, 2t+1) to the B fragment (row
-            // t + 4 ks, column g)
-            const int src = (t + 4 * ks) * 4 + (g >> 1);
-            const double b0 = __shfl_sync(0xffffffffu, y0, src), b1 = __shfl_sync(0xffffffffu, y1, src);
-            dmma(r0, r1, fragA(X, 8 * p, 8 * p, ks), (g & 1) ? b1 : b0);
-        }
-        X[tix<double>(8 * p + g, 8 * j + 2 * t)] = -r0;
-        X[tix<double>(8 * p + g, 8 * j + 2 * t + 1)] = -r1;
-    };
-    if (wid == 0) chol8(D, X, 0, pivtol, status, colbase, w);
-    bar_consumers();
-    for (int p = 0; p < nb; p++) {
-        if (wid == 0) {
-            if (p + 1 < nb) {
-                const int i = p + 1;
-                double d0, d1;
-                panel(i, p, d0, d1);
-                scr[(2 * t) * 8 + g] = d0;           // L_ip(g, k) at scr[8 k + g]
+                for (int ks = 0; ks < 2; ks++) dmma(d0, d1, D[at.nn(8 * i, 8 * p, ks)], xp[ks]);
+                scr[(2 * t) * 8 + g] = d0;                   // L_ip(g, k) at scr[8 k + g]
                 scr[(2 * t + 1) * 8 + g] = d1;
                 __syncwarp();
                 double u0 = 0.0, u1 = 0.0;
@@ -392,36 +406,97 @@ SPX_DEV void chol_inv64(double *D, double *X, double *scr, int w, double pivtol,
                     const double f = scr[(4 * ks + t) * 8 + g];
                     dmma(u0, u1, f, f);
                 }
-                D[tix<double>(8 * i + g, 8 * i + 2 * t)] -= u0;
-                D[tix<double>(8 * i + g, 8 * i + 2 * t + 1)] -= u1;
+                D[c0] = e0 - u0;
+                D[c1] = e1 - u1;
                 __syncwarp();
-                chol8(D, X, 8 * i, pivtol, status, colbase, w);
             }
-        } else {
-            // the panel: L_ip transposed into block (p, i)
-            for (int i = p + 1 + (wid - 1); i < nb; i += 3) {
-                double d0, d1;
-                panel(i, p, d0, d1);
-                D[tix<double>(8 * p + 2 * t, 8 * i + g)] = d0;
-                D[tix<double>(8 * p + 2 * t + 1, 8 * i + g)] = d1;
+            chol8(D, X, 8 * i, pivtol, status, colbase, w);
+        }
+        if (wid > 0 && p >= 0 && p + 1 < nb) {
+            // the panel: rows i = p + wid + 3 q, L_ip transposed into block (p, i)
+            double d[3][2];
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const int i = p + wid + 3 * q;
+                d[q][0] = d[q][1] = 0.0;
+                if (i < nb)
+#pragma unroll
+                    for (int ks = 0; ks < 2; ks++) dmma(d[q][0], d[q][1], D[at.nn(8 * i, 8 * p, ks)], xp[ks]);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const int i = p + wid + 3 * q;
+                if (i < nb) {
+                    D[tix<double>(8 * p + 2 * t, 8 * i + g)] = d[q][0];
+                    D[tix<double>(8 * p + 2 * t + 1, 8 * i + g)] = d[q][1];
+                }
             }
             asm volatile("bar.sync 2, 96;" ::: "memory");
-            // trailing blocks (i, j), p < j <= i, without (p+1, p+1), then row
-            // p of the inverse
-            int task = 0;
-            for (int j = p + 1; j < nb; j++)
-                for (int i = j + (j == p + 1); i < nb; i++, task++) {
-                    if (task % 3 != wid - 1) continue;
-                    double u0 = 0.0, u1 = 0.0;
+            // trailing blocks (i, j), p < j <= i, without (p+1, p+1): block
+            // rows from the bottom, dealt to the warps, all blocks of a row
+            // together
+            for (int i = nb - wid; i > p + 1; i -= 3) {
+                double a[2];
+#pragma unroll
+                for (int ks = 0; ks < 2; ks++) a[ks] = D[at.tn(8 * p, 8 * i, ks)];
+#pragma unroll 1
+                for (int j0 = p + 1; j0 <= i; j0 += 4) {
+                    double u[4][2];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        u[q][0] = u[q][1] = 0.0;
+                        if (j0 + q > i) break;
+#pragma unroll
+                        for (int ks = 0; ks < 2; ks++)
+                            dmma(u[q][0], u[q][1], a[ks], D[at.tn(8 * p, 8 * (j0 + q), ks)]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (j0 + q > i) break;
+#pragma unroll
+                        for (int z = 0; z < 2; z++) D[at.cc(8 * i, 8 * (j0 + q), z)] -= u[q][z];
+                    }
+                }
+            }
+        }
+        // row p of the inverse, a few blocks j a warp: X_pj = -X_pp sum_{j <= k < p}
+        // L_pk X_kj, with L_pk(m, s) at D(8k + s, 8p + m); warp 0 joins in
+        // once its chain is through
+        const bool all = p + 1 == nb;
+        const int nw = all ? 4 : 3, me = all ? wid : wid - 1;
+        if (me >= 0 && p > 0) {
+            double y[3][2];
+#pragma unroll
+            for (int q = 0; q < 3; q++) y[q][0] = y[q][1] = 0.0;
+            for (int k = 0; k < p; k++) {
+                double a[2];
+#pragma unroll
+                for (int ks = 0; ks < 2; ks++) a[ks] = D[at.tn(8 * k, 8 * p, ks)];
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    if (me + nw * q > k) break;
 #pragma unroll
                     for (int ks = 0; ks < 2; ks++)
-                        dmma(u0, u1, D[tix<double>(8 * p + 4 * ks + t, 8 * i + g)],
-                             D[tix<double>(8 * p + 4 * ks + t, 8 * j + g)]);
-                    D[tix<double>(8 * i + g, 8 * j + 2 * t)] -= u0;
-                    D[tix<double>(8 * i + g, 8 * j + 2 * t + 1)] -= u1;
+                        dmma(y[q][0], y[q][1], a[ks], X[at.tn(8 * k, 8 * (me + nw * q), ks)]);
                 }
-            for (int j = 0; j < p; j++, task++)
-                if (task % 3 == wid - 1) xrow(p, j);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const int j = me + nw * q;
+                if (j >= p) break;
+                double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+                for (int ks = 0; ks < 2; ks++) {
+                    // accumulator (row g, columns 2t, 2t+1) to the B fragment
+                    // (row t + 4 ks, column g)
+                    const int src = (t + 4 * ks) * 4 + (g >> 1);
+                    const double b0 = __shfl_sync(0xffffffffu, y[q][0], src);
+                    const double b1 = __shfl_sync(0xffffffffu, y[q][1], src);
+                    dmma(r0, r1, xp[ks], (g & 1) ? b1 : b0);
+                }
+                X[at.cc(8 * p, 8 * j, 0)] = -r0;
+                X[at.cc(8 * p, 8 * j, 1)] = -r1;
+            }
         }
         bar_consumers();
     }
@@ -478,7 +553,7 @@ SPX_DEV void fproduce(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
             const int k1 = tk.kind == FK_INV ? I : f.nkb;
             for (int k = J; k < k1; k++) {
                 need(f.lflag(I, k));
-                need(k == J ? f.lflag(J, J) : f.xflag(J, k));
+                need(f.xflag(J, k));
                 fence_async_all();
                 produce_chunks(a, sh, pp, Fp + f.ltile(I, k), Fp + f.xtile(J, k), f.width(k));
             }
@@ -530,19 +605,34 @@ SPX_DEV void store_diag(FShared &sh, const Acc &acc, int w, int m0, int n0) {
     });
 }
 
-// X_JJ (w x w lower, zero elsewhere) to the panel, and to tile storage as it
-// is and transposed
-SPX_DEV void write_inverse(const FactorArgs &a, const double *X, int w, Real *G, int at, int c,
-                           Real *L, Real *Xt) {
+// X_JJ (w x w lower, zero elsewhere) to tile storage; first of all, because
+// the chain waits for it (pairs of entries: the layouts of X and of an FP64
+// tile are the same)
+SPX_DEV void write_inverse_tile(const double *X, int w, Real *L) {
+    for (int t = threadIdx.x; t < FT / 2 * round4(w); t += kFConsumers) {
+        const int j = t >> 5;
+        if constexpr (sizeof(Real) == 8) {
+            const int i = (2 * (t & 31)) ^ ((j & 3) << 2);       // even, as the XOR is
+            double2 v = reinterpret_cast<const double2 *>(X)[t];
+            if (!(i >= j && i < w && j < w)) v.x = 0.0;
+            if (!(i + 1 >= j && i + 1 < w && j < w)) v.y = 0.0;
+            reinterpret_cast<double2 *>(L)[t] = v;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int i = 2 * (t & 31) + e;
+                L[tix<Real>(i, j)] = (Real)((i >= j && i < w && j < w) ? X[tix<double>(i, j)] : 0.0);
+            }
+        }
+    }
+}
+// and to the panel, and transposed to the inverse's tile storage (if any)
+SPX_DEV void write_inverse(const double *X, int w, Real *G, int at, int c, Real *Xt) {
     const int w4 = round4(w);
     for (int t = threadIdx.x; t < FT * w4; t += kFConsumers) {
         const int i = t & (FT - 1), j = t >> 6;
-        const Real lo = (Real)((j < w && i < w && i >= j) ? X[tix<double>(i, j)] : 0.0);
-        if (j < w && i < w && i >= j) G[gix(at + i, at + j, c)] = lo;
-        if (L) {
-            L[tix<Real>(i, j)] = lo;
-            Xt[tix<Real>(i, j)] = (Real)((i < w && j < w && j >= i) ? X[tix<double>(j, i)] : 0.0);
-        }
+        if (j < w && i < w && i >= j) G[gix(at + i, at + j, c)] = (Real)X[tix<double>(i, j)];
+        if (Xt) Xt[tix<Real>(i, j)] = (Real)((i < w && j < w && j >= i) ? X[tix<double>(j, i)] : 0.0);
     }
 }
 
@@ -590,58 +680,11 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
     // tiles of the front proper start with their assembly
     if (nd.b.y > 0 && tid == 0) fwait(a.upd + tk.s, nd.b.w, a.err);
     if (nd.b.y > 0) bar_consumers();
-    if (tk.kind == FK_SMALL) {
-        double *P = X + FT * FT;
-        const int w = f.c, nb = f.r - f.c, w4 = round4(w);
-        const int mi = min(4, (nb - m0 + 7) >> 3), nj = min(4, (w - n0 + 7) >> 3);
-        assemble(a, nd, sh.S, 0, 0, 0, w, 0, w, true);
-        store_diag(sh, acc, w, m0, n0);
-        if (nb > 0) assemble(a, nd, P, 1, 0, w, nb, 0, w, true);
-        else bar_consumers();
-        chol_inv64(sh.S, X, sh.scratch[0], w, a.params[1], a.status, nd.a.x);
-        // zero above the diagonal blocks, for the products
-        for (int t = tid; t < FT * w4; t += kFConsumers) {
-            const int i = t & (FT - 1), j = t >> 6;
-            if (i < j || i >= w || j >= w) X[tix<double>(i, j)] = 0.0;
-        }
-        bar_consumers();
-        write_inverse(a, X, w, Gp, 0, f.c, nullptr, nullptr);
-        if (nb > 0) {
-            mma_cols(acc, P, X, w4 >> 2, m0, n0, mi, nj);          // L21 = P X^T
-            bar_consumers();
-            acc_each(acc, m0, n0, [&](int m, int n, double v) {
-                // FP32 storage rounds L21 as a stored tile would be
-                if (n < w4) P[tix<double>(m, n)] = n < w ? (double)(Real)v : 0.0;
-            });
-            // S(n, k) = X(k, n): the second operand of W = L21 X
-            for (int t = tid; t < FT * w4; t += kFConsumers) {
-                const int n = t & (FT - 1), k = t >> 6;
-                sh.S[tix<double>(n, k)] = (n < w && k < w && k >= n) ? (double)(Real)X[tix<double>(k, n)] : 0.0;
-            }
-            bar_consumers();
-            acc_zero(acc);
-            mma_cols(acc, P, sh.S, w4 >> 2, m0, n0, mi, nj);
-            acc_each(acc, m0, n0, [&](int m, int n, double v) {
-                if (m < nb && n < w) Gp[gix(w + m, n, f.c)] = (Real)v;
-            });
-            bar_consumers();
-            assemble(a, nd, sh.S, 1, 1, w, nb, w, nb, false);
-            acc_zero(acc);
-            const int nj2 = min(4, (nb - n0 + 7) >> 3);
-            mma_cols(acc, P, P, w4 >> 2, m0, n0, mi, nj2);
-            Real *U = a.F + nd.p.y;
-            acc_each(acc, m0, n0, [&](int m, int n, double v) {
-                if (m < nb && n <= m) U[tix<Real>(m, n)] = (Real)(sh.S[tix<double>(m, n)] - v);
-            });
-            if (nd.b.x >= 0) publish(a.upd + nd.b.x);
-        }
-        fence_async_all();           // the ring's memory goes back to the bulk copies
-        return;
-    }
+    const bool small = tk.kind == FK_SMALL;
     const int ra = f.start(I), ca = f.start(J), h = f.width(I), w = f.width(J);
     const int mi = min(4, (h - m0 + 7) >> 3), nj = min(4, (w - n0 + 7) >> 3);
     assemble(a, nd, sh.S, I, J, ra, h, ca, w, J < f.nkb);
-    const int k1 = min(J, f.nkb);
+    const int k1 = small ? 0 : min(J, f.nkb);
     for (int k = 0; k < k1; k++)
         consume_block<false, false>(sh, pp, acc, I == J, f.width(k), m0, n0, mi, nj, a.err);
     if (tk.kind == FK_SCHUR) {
@@ -670,13 +713,59 @@ SPX_DEV void fconsume(const FactorArgs &a, FShared &sh, FPipe &pp, const FTask &
         publish(fl + f.lflag(I, J));
         return;
     }
-    // FK_DIAG: the ring is drained (this task has no further chunks)
+    // FK_DIAG, FK_SMALL: the ring is drained (the task has no further chunks)
+    // and holds X and, for FK_SMALL, the rows below
+    double *P = X + FT * FT;
+    const int nb = f.r - f.c, w4 = round4(w);
     store_diag(sh, acc, w, m0, n0);
-    bar_consumers();
+    if (small && nb > 0) assemble(a, nd, P, 1, 0, w, nb, 0, w, true);
+    else bar_consumers();
     chol_inv64(sh.S, X, sh.scratch[0], w, a.params[1], a.status, nd.a.x + ca);
-    write_inverse(a, X, w, Gp, ca, f.c, Fp + f.ltile(J, J),
-                  Fp + f.xtile(J, J));
-    publish(fl + f.lflag(J, J));     // (also orders the ring's reuse by bulk copies)
+    if (!small) {
+        write_inverse_tile(X, w, Fp + f.ltile(J, J));
+        publish(fl + f.lflag(J, J));
+        write_inverse(X, w, Gp, ca, f.c, Fp + f.xtile(J, J));
+        publish(fl + f.xflag(J, J)); // (also orders the ring's reuse by bulk copies)
+        return;
+    }
+    // zero above the diagonal blocks, for the products
+    for (int t = tid; t < FT * w4; t += kFConsumers) {
+        const int i = t & (FT - 1), j = t >> 6;
+        if (i < j || i >= w || j >= w) X[tix<double>(i, j)] = 0.0;
+    }
+    bar_consumers();
+    write_inverse(X, w, Gp, 0, f.c, nullptr);
+    if (nb > 0) {
+        const int mb = min(4, (nb - m0 + 7) >> 3), nb2 = min(4, (nb - n0 + 7) >> 3);
+        acc_zero(acc);
+        mma_cols(acc, P, X, w4 >> 2, m0, n0, mb, nj);              // L21 = P X^T
+        bar_consumers();
+        acc_each(acc, m0, n0, [&](int m, int n, double v) {
+            // FP32 storage rounds L21 as a stored tile would be
+            if (n < w4) P[tix<double>(m, n)] = n < w ? (double)(Real)v : 0.0;
+        });
+        // S(n, k) = X(k, n): the second operand of W = L21 X
+        for (int t = tid; t < FT * w4; t += kFConsumers) {
+            const int n = t & (FT - 1), k = t >> 6;
+            sh.S[tix<double>(n, k)] = (n < w && k < w && k >= n) ? (double)(Real)X[tix<double>(k, n)] : 0.0;
+        }
+        bar_consumers();
+        acc_zero(acc);
+        mma_cols(acc, P, sh.S, w4 >> 2, m0, n0, mb, nj);
+        acc_each(acc, m0, n0, [&](int m, int n, double v) {
+            if (m < nb && n < w) Gp[gix(w + m, n, f.c)] = (Real)v;
+        });
+        bar_consumers();
+        assemble(a, nd, sh.S, 1, 1, w, nb, w, nb, false);
+        acc_zero(acc);
+        mma_cols(acc, P, P, w4 >> 2, m0, n0, mb, nb2);
+        Real *U = a.F + nd.p.y;
+        acc_each(acc, m0, n0, [&](int m, int n, double v) {
+            if (m < nb && n <= m) U[tix<Real>(m, n)] = (Real)(sh.S[tix<double>(m, n)] - v);
+        });
+        if (nd.b.x >= 0) publish(a.upd + nd.b.x);
+    }
+    fence_async_all();               // the ring's memory goes back to the bulk copies
 }
 
 // After a pivot failure the remaining tasks do no work but still publish, so
@@ -686,7 +775,7 @@ SPX_DEV void fskip(const FactorArgs &a, const FTask &tk, const FNode &nd) {
     const FGeo f = geo_of(nd);
     int *fl = a.flags + nd.f.x;
     switch (tk.kind) {
-        case FK_DIAG:
+        case FK_DIAG: add_release(fl + f.xflag(tk.J, tk.J), 1);
         case FK_ROWS: add_release(fl + f.lflag(tk.I, tk.J), 1); break;
         case FK_INV: add_release(fl + f.xflag(tk.J, tk.I), 1); break;
         case FK_SMALL: if (f.r == f.c) break;   // no update matrix
@@ -695,6 +784,7 @@ SPX_DEV void fskip(const FactorArgs &a, const FTask &tk, const FNode &nd) {
     }
 }
 
+// (168 registers a thread: ten warps an SM put three on some sub-partitions)
 __global__ void __launch_bounds__(kFThreads, 2) mf_factor(FactorArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     FShared &sh = *reinterpret_cast<FShared *>(smem_raw);

@@ -12,6 +12,7 @@
 #include "../host/parallel.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <new>
 
@@ -120,14 +121,17 @@ static_assert(sizeof(FTaskH) == sizeof(FTask), "factor task layout");
 
 // The factor's nodes, tile storage (in Reals) and task queue.
 //
-// A task's key is an estimate (us) of the path from it to the end of the
-// root: a column block of a front's diagonal chain costs kStep, and a front
-// kFront for its assembly and hand-over.  Tasks run in decreasing key order,
-// equal keys in the order they were made, which puts every task after the
-// ones it waits for: a front starts below its children's update tiles, a
-// column block below the one before it, rows below their diagonal tile.
-// Inverse tiles follow two column blocks behind the chain; W tiles, which no
-// factor task waits for, fill the middle of the parent's chain.
+// A task's key is an estimate of how early it can run (quarter microseconds):
+// the longest path of column blocks below it, kStep for a column block of a
+// front's diagonal chain and kFront for a front's assembly and hand-over.
+// Tasks run in increasing key order, equal keys in the order they were made.
+// The key grows along every dependency, which puts every task after the ones
+// it waits for: a front starts after its children's update tiles, a column
+// block after the one before it, rows after their diagonal tile, inverse
+// tiles two column blocks behind the chain, W tiles last.  Starting the
+// longest chains first instead (by the path above a task) or a mix of the two
+// measured the same to 3 % (48^3 4.60 against 4.44 ms): the blocks held by
+// tiles that wait for a chain cost what the chains gain.
 static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
                               std::vector<FNodeH> &node, std::vector<FChildH> &child,
                               std::vector<int32_t> &cbnd, std::vector<FTaskH> &tasks,
@@ -135,7 +139,7 @@ static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
     constexpr int kStep = 15, kFront = 12, kRes = 4;
     const int32_t ns = S.nsuper;
     int64_t off = 0, nfl = 0;
-    std::vector<int32_t> start(ns, 0);           // key of a front's first task
+    std::vector<int64_t> early(ns, 0);           // key of a front's first task
     auto r4 = [](int64_t v) { return (v + 3) & ~(int64_t)3; };
     auto is_small = [&](int32_t s) { return node[s].nkb == 1 && node[s].nt <= 2; };
     for (int32_t s = 0; s < ns; s++) {
@@ -167,10 +171,9 @@ static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
             off += (int64_t)FT * FT * ((nu - 1) * nu - (nu - 1) * (nu - 2) / 2) + FT * wl4;
         }
     }
-    for (int32_t s = ns - 1; s >= 0; s--) {
-        const FNodeH &m = node[s];
-        start[s] = kRes * (kFront + kStep * m.nkb) + (m.parent < 0 ? 0 : start[m.parent]);
-    }
+    auto span = [&](int32_t s) { return (int64_t)kRes * (kFront + kStep * node[s].nkb); };
+    for (int32_t s = 0; s < ns; s++)
+        if (node[s].parent >= 0) early[node[s].parent] = std::max(early[node[s].parent], early[s] + span(s));
     int64_t ntask = 0, nbnd = 0;
     for (int32_t s = 0; s < ns; s++) {
         const FNodeH &m = node[s];
@@ -205,8 +208,10 @@ static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
     std::vector<int32_t> key;
     t.reserve(ntask);
     key.reserve(ntask);
-    int32_t kmin = 0, kmax = 0;
-    auto emit = [&](int kind, int s, int I, int J, int k) {
+    int32_t kmin = INT32_MAX, kmax = INT32_MIN;
+    // `at`: quarter microseconds after the front's first task
+    auto emit = [&](int kind, int s, int I, int J, int64_t at) {
+        const int32_t k = (int32_t)(early[s] + at);
         t.push_back({kind, s, I, J});
         key.push_back(k);
         kmin = std::min(kmin, k);
@@ -215,33 +220,32 @@ static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
     for (int32_t s = 0; s < ns; s++) {
         const FNodeH &m = node[s];
         if (is_small(s)) {
-            emit(FK_SMALL, s, 0, 0, start[s]);
+            emit(FK_SMALL, s, 0, 0, 0);
             continue;
         }
-        const int up = m.parent < 0 ? 0 : start[m.parent];
-        const int tp = m.parent < 0 ? 0 : kRes * (kFront + kStep * node[m.parent].nkb);
         for (int J = 0; J < m.nkb; J++) {
-            emit(FK_DIAG, s, J, J, start[s] - kRes * kStep * J);
-            for (int I = J + 1; I < m.nt; I++) emit(FK_ROWS, s, I, J, start[s] - kRes * (kStep * J + 4));
+            emit(FK_DIAG, s, J, J, kRes * kStep * J);
+            for (int I = J + 1; I < m.nt; I++) emit(FK_ROWS, s, I, J, kRes * (kStep * J + 4));
         }
         for (int J = m.nkb; J < m.nt; J++)
-            for (int I = J; I < m.nt; I++) emit(FK_SCHUR, s, I, J, up + kRes * 8);
+            for (int I = J; I < m.nt; I++) emit(FK_SCHUR, s, I, J, kRes * (kStep * m.nkb + 4));
         for (int i = 1; i < m.nkb; i++)
-            for (int j = 0; j < i; j++) emit(FK_INV, s, i, j, start[s] - kRes * (kStep * i + 20));
+            for (int j = 0; j < i; j++) emit(FK_INV, s, i, j, kRes * (kStep * i + kStep + 5));
+        const int64_t tp = m.parent < 0 ? 0 : span(m.parent);
         for (int J = 0; J < m.nkb; J++)
-            for (int I = m.nkb; I < m.nt; I++) emit(FK_WMUL, s, I, J, up - kRes * 2 - tp / 2);
+            for (int I = m.nkb; I < m.nt; I++) emit(FK_WMUL, s, I, J, span(s) + kRes * (kStep + 6) + tp / 2);
     }
     const int64_t range = (int64_t)kmax - kmin + 1;
     tasks.resize(t.size());
     if (range <= 4 * (int64_t)t.size() + 65536) {
         std::vector<int32_t> cnt(range + 1, 0);
-        for (int32_t k : key) cnt[kmax - k + 1]++;
+        for (int32_t k : key) cnt[k - kmin + 1]++;
         for (int64_t q = 0; q < range; q++) cnt[q + 1] += cnt[q];
-        for (size_t i = 0; i < t.size(); i++) tasks[cnt[kmax - key[i]]++] = t[i];
+        for (size_t i = 0; i < t.size(); i++) tasks[cnt[key[i] - kmin]++] = t[i];
     } else {
         std::vector<int32_t> ord(t.size());
         for (size_t i = 0; i < t.size(); i++) ord[i] = (int32_t)i;
-        std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key[x] > key[y]; });
+        std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key[x] < key[y]; });
         for (size_t i = 0; i < t.size(); i++) tasks[i] = t[ord[i]];
     }
     *storage = off;
@@ -486,7 +490,8 @@ template <> MultifrontalPlanT<Real>::~MultifrontalPlanT() { release(0); }
 template <> void MultifrontalPlanT<Real>::release(cudaStream_t st) {
     void **ptrs[] = {(void **)&d_params_, (void **)&d_perm_, (void **)&d_rows_, (void **)&d_relmap_,
                      (void **)&d_cbnd_, (void **)&d_fnode_, (void **)&d_fchild_, (void **)&d_ftask_,
-                     (void **)&d_fsync_, (void **)&d_acolptr_, (void **)&d_atpos_, (void **)&d_asrc_,
+                     (void **)&d_fsync_, (void **)&d_acolptr_, (void **)&d_atpos_, (void **)&d_acolj_,
+                     (void **)&d_asrc_,
                      (void **)&d_front_, (void **)&d_G_, (void **)&d_vtask_, (void **)&d_btask_,
                      (void **)&d_cptr_, (void **)&d_cidx_, (void **)&d_sync_, (void **)&d_sval_[0],
                      (void **)&d_sval_[1], (void **)&d_sval_[2], (void **)&d_sval_[3],
@@ -528,7 +533,8 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         // bounds are independent of the task lists: they are built on side
         // threads while this thread builds the factor and solve task lists.
         std::vector<int32_t> acolptr(n + 1, 0);
-        std::vector<int32_t> atpos, asrc;
+        std::vector<int32_t> atpos, acolj, asrc;
+        std::atomic<int> dup{0};
         std::vector<int32_t> cptr(nrows_total_ + 1, 0), cidx;
         std::vector<int32_t> cbnd;
         std::vector<FNodeH> fnode(ns);
@@ -551,6 +557,7 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
             });
             for (int32_t j = 0; j < n; j++) acolptr[j + 1] += acolptr[j];
             atpos.resize(acolptr[n]);
+            acolj.resize(acolptr[n]);
             asrc.resize(acolptr[n]);
             parallel_ranges(ns, 128, [&](int64_t lo, int64_t hi) {
                 std::vector<int32_t> pos(n, -1);
@@ -568,7 +575,12 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
                         }
                         std::sort(tmp.begin(), tmp.end());
                         int32_t d = acolptr[j];
-                        for (auto &e : tmp) { atpos[d] = e.first; asrc[d] = e.second; d++; }
+                        for (auto &e : tmp) {
+                            if (d > acolptr[j] && atpos[d - 1] == e.first) dup = 1;
+                            atpos[d] = e.first;
+                            acolj[d] = j;
+                            asrc[d++] = e.second;
+                        }
                     }
                     for (int64_t t = r0; t < r1; t++) pos[S.rows[t]] = -1;
                 }
@@ -640,7 +652,9 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         rc = rc ? rc : dupload(&d_relmap_, S.relmap, (size_t)nrows_total_, st);
         rc = rc ? rc : dupload(&d_acolptr_, acolptr.data(), n + 1, st);
         rc = rc ? rc : dupload(&d_atpos_, atpos.data(), atpos.size(), st);
+        rc = rc ? rc : dupload(&d_acolj_, acolj.data(), acolj.size(), st);
         rc = rc ? rc : dupload(&d_asrc_, asrc.data(), asrc.size(), st);
+        dup_ = dup;
         // per column count 1, 8, 16, 24, 32: queue, blocks gone, copy in use;
         // then the error word
         rc = rc ? rc : dmalloc(&d_sync_, 16, st);
@@ -707,7 +721,9 @@ template <> int MultifrontalPlanT<Real>::factorize(const double *d_val, double s
     a.cbnd = d_cbnd_;
     a.acolptr = d_acolptr_;
     a.atpos = d_atpos_;
+    a.acolj = d_acolj_;
     a.asrc = d_asrc_;
+    a.dup = dup_;
     a.val = d_val;
     a.params = d_params_;
     a.F = d_front_;

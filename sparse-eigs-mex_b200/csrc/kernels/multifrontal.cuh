@@ -86,7 +86,9 @@ private:
     int32_t *d_perm_ = nullptr, *d_rows_ = nullptr, *d_relmap_ = nullptr;
     int32_t *d_acolptr_ = nullptr;   // [n+1] assembly entries per new column
     int32_t *d_atpos_ = nullptr;     // row position within the front
+    int32_t *d_acolj_ = nullptr;     // column (new numbering)
     int32_t *d_asrc_ = nullptr;      // index into the CSR values
+    int dup_ = 0;                    // some entry of A is stored more than once
     int32_t *d_cbnd_ = nullptr;      // child bounds per parent 64-row tile
     // factor: per-supernode metadata, child records, tile task queue, flags
     void *d_fnode_ = nullptr, *d_fchild_ = nullptr, *d_ftask_ = nullptr;
