@@ -16,6 +16,7 @@
 #include "kernels/dense_lu.cuh"
 #include "kernels/dense_eig.cuh"
 #include "kernels/seg_lanczos.cuh"
+#include "chain.cuh"
 #include "counters.h"
 #include "host/syev_host.h"
 
@@ -470,6 +471,7 @@ struct LanczosBufs {
 
 __global__ void thsave_kernel(const double *theta, const int *ord, int t, double *thsave,
                               int nret) {
+    chain_begin();
     thsave[nret] = theta[ord[t]];
 }
 
@@ -777,8 +779,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
                 orth_block(b, b.Vn, t, dst, nullptr, st);
                 launch_flag_if_below(b.nrm2, 1e-20, b.dflag, st);
                 normalise(n, dst, b.nrm2, dst, st);
-                thsave_kernel<<<1, 1, 0, st>>>(b.theta, b.ord, t, b.thsave, t);
-                note_launch();
+                launch_chained(thsave_kernel, 1, 1, 0, st, b.theta, b.ord, t, b.thsave, t);
             }
             copy_async(h_rflag, b.dflag, sizeof(int), cudaMemcpyDeviceToHost, st);
             tm.end(tk, &ms_ritz);
@@ -798,8 +799,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
                 if (int e = read_nrm(&nv)) return e;
                 if (nv < 1e-10) continue;
                 normalise(n, dst, b.nrm2, dst, st);
-                thsave_kernel<<<1, 1, 0, st>>>(b.theta, b.ord, t, b.thsave, nret);
-                note_launch();
+                launch_chained(thsave_kernel, 1, 1, 0, st, b.theta, b.ord, t, b.thsave, nret);
                 nret++;
             }
             tm.end(tk, &ms_ritz);

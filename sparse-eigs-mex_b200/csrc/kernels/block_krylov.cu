@@ -4,6 +4,7 @@
 // the block W (n x b); the small dense parts (b x b Cholesky and inverse)
 // run in one warp.
 #include "block_krylov.cuh"
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(kTbThreads) tsb_tn_part_kernel(
     // (cp.async, 8 bytes each, zero-filled past the range) are in flight
     // while chunk i is multiplied
     extern __shared__ double dsm[];
+    chain_begin();
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, gq = lane >> 2, tq = lane & 3;
     const int nmt = (m + 7) >> 3, nnt = (b + 7) >> 3, ncol = m + b;
     double acc[2][4][2];
@@ -132,6 +134,7 @@ __global__ void __launch_bounds__(kTbThreads) tsb_fused_part_kernel(
         int ldh1, double *__restrict__ W, int64_t ldw, int b, int rows_per_part,
         double *__restrict__ part) {
     extern __shared__ double dsm[];
+    chain_begin();
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, gq = lane >> 2, tq = lane & 3;
     if (MODE == kMulGram) m = 0;                          // no V: the chunk is W alone
     const int nnt = (b + 7) >> 3, ncol = m + b;
@@ -249,6 +252,7 @@ constexpr int kRedSlices = 8;
 __global__ void __launch_bounds__(32 * kRedSlices) tsb_tn_reduce_kernel(
         int m, int b, int nparts, const double *__restrict__ part, double *H, int ldh, int mode) {
     __shared__ double sl[kRedSlices][33];
+    chain_begin();
     const int lo = threadIdx.x & 31, sli = threadIdx.x >> 5;
     const int o = blockIdx.x * 32 + lo;
     const bool live = o < m * kBlockMaxB;
@@ -280,6 +284,7 @@ __global__ void __launch_bounds__(kTbThreads) tsb_rows_kernel(const double *A, i
                                                               int K, const double *Bm, int ldb,
                                                               double *W, int64_t ldw, int b) {
     __shared__ double Bs[kBlockMaxM][kVS];
+    chain_begin();
     const int nks = (K + 3) >> 2;
     for (int e = threadIdx.x; e < nks * 4 * kVS; e += kTbThreads) {
         const int k = e / kVS, j = e % kVS;
@@ -331,6 +336,7 @@ __global__ void block_chol_kernel(int b, const double *G, int ldg, double *Rinv,
                                   double rel_floor, int *status) {
     __shared__ double R[kBlockMaxB][kBlockMaxB + 1];   // R[i][j], upper
     __shared__ double d[kBlockMaxB];
+    chain_begin();
     const int j = threadIdx.x;
     unsigned dep = 0;
     // column scales: unit diagonal after scaling
@@ -555,11 +561,11 @@ void launch_tsb_tn(const double *V, int64_t ldv, int n, int m, const double *W, 
                              (int)(sizeof(double) * 2 * (kBlockMaxM + kBlockMaxB) * kVS));
         attr = true;
     }
-    tsb_tn_part_kernel<<<np, kTbThreads, smem, st>>>(V, ldv, n, m, W, ldw, b, rows, bs.part);
+    launch_chained(tsb_tn_part_kernel, np, kTbThreads, smem, st, V, ldv, n, m, W, ldw, b, rows,
+                   bs.part);
     const int outs = m * kBlockMaxB;
-    tsb_tn_reduce_kernel<<<(outs + 31) / 32, 32 * kRedSlices, 0, st>>>(m, b, np, bs.part, H, ldh,
-                                                                       mode);
-    note_launch(2);
+    launch_chained(tsb_tn_reduce_kernel, (outs + 31) / 32, 32 * kRedSlices, 0, st, m, b, np, bs.part,
+                   H, ldh, mode);
 }
 
 namespace {
@@ -584,13 +590,12 @@ void launch_fused(const double *V, int64_t ldv, int n, int m, const double *H1, 
                                                      kBlockMaxM * (kBlockMaxB + 4))));
         attr = true;
     }
-    tsb_fused_part_kernel<MODE><<<np, kTbThreads, smem, st>>>(V, ldv, n, mm, H1, ldh1, W, ldw, b,
-                                                               rows, bs.part);
+    launch_chained(tsb_fused_part_kernel<MODE>, np, kTbThreads, smem, st, V, ldv, n, mm, H1, ldh1, W,
+                   ldw, b, rows, bs.part);
     const int pm = MODE == kSubTn ? m : b;
     const int outs = pm * kBlockMaxB;
-    tsb_tn_reduce_kernel<<<(outs + 31) / 32, 32 * kRedSlices, 0, st>>>(pm, b, np, bs.part, H2, ldh2,
-                                                                       mode);
-    note_launch(2);
+    launch_chained(tsb_tn_reduce_kernel, (outs + 31) / 32, 32 * kRedSlices, 0, st, pm, b, np, bs.part,
+                   H2, ldh2, mode);
 }
 }  // namespace
 
@@ -618,33 +623,29 @@ void launch_tsb_nn_sub(const double *V, int64_t ldv, int n, int m, const double 
                        double *W, int64_t ldw, int b, cudaStream_t st) {
     if (m <= 0 || b <= 0) return;
     const int rows = kTbThreads / 4;
-    tsb_rows_kernel<true><<<(n + rows - 1) / rows, kTbThreads, 0, st>>>(V, ldv, n, m, H, ldh, W,
-                                                                        ldw, b);
-    note_launch();
+    launch_chained(tsb_rows_kernel<true>, (n + rows - 1) / rows, kTbThreads, 0, st, V, ldv, n, m, H,
+                   ldh, W, ldw, b);
 }
 
 void launch_block_chol(int b, const double *G, int ldg, double *Rinv, double abs_floor,
                        double rel_floor, int *status, cudaStream_t st) {
-    block_chol_kernel<<<1, 32, 0, st>>>(b, G, ldg, Rinv, abs_floor, rel_floor, status);
-    note_launch();
+    launch_chained(block_chol_kernel, 1, 32, 0, st, b, G, ldg, Rinv, abs_floor, rel_floor, status);
 }
 
 void launch_tsb_right_mul(int n, int b, double *W, int64_t ldw, const double *Rinv,
                           cudaStream_t st) {
     if (b <= 0) return;
     const int rows = kTbThreads / 4;
-    tsb_rows_kernel<false><<<(n + rows - 1) / rows, kTbThreads, 0, st>>>(W, ldw, n, b, Rinv, b, W,
-                                                                         ldw, b);
-    note_launch();
+    launch_chained(tsb_rows_kernel<false>, (n + rows - 1) / rows, kTbThreads, 0, st, W, ldw, n, b,
+                   Rinv, b, W, ldw, b);
 }
 
 void launch_tsb_right_mul_into(int n, int K, const double *X, int64_t ldx, const double *S,
                                int lds, double *W, int64_t ldw, int b, cudaStream_t st) {
     if (b <= 0 || K <= 0) return;
     const int rows = kTbThreads / 4;
-    tsb_rows_kernel<false><<<(n + rows - 1) / rows, kTbThreads, 0, st>>>(X, ldx, n, K, S, lds, W,
-                                                                         ldw, b);
-    note_launch();
+    launch_chained(tsb_rows_kernel<false>, (n + rows - 1) / rows, kTbThreads, 0, st, X, ldx, n, K, S,
+                   lds, W, ldw, b);
 }
 
 void launch_block_refine_residual(int n, const int32_t *rowptr, const int32_t *col,

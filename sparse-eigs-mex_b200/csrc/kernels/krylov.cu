@@ -8,6 +8,7 @@
 // orth_block (:122-132), dnrm2/dscal/ddot (:189-191, :209, :223, :251-257),
 // dgemv N for Ritz vectors (:250, :278), dsyev (:236) and rand_vec (:49-54).
 #include "krylov.cuh"
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 
@@ -24,7 +25,9 @@ namespace spx {
 // a pair of values (16 bytes) and a pair of column indices (8 bytes) per
 // thread and step, after at most one leading entry that puts the pairs on
 // their 16-byte boundary -- and each thread then sums its own row from
-// shared memory (CSR-stream); otherwise a warp walks each row.
+// shared memory (CSR-stream); otherwise a warp walks each row.  Bound by the
+// matrix's bytes, if enough loads are in flight: 100^3 grid, 7 entries a row
+// (104 MB), 39 us with one pair at a time, 31 with four.
 constexpr int kSpmvRows = 128;
 constexpr int kSpmvCap = 2048;
 
@@ -33,6 +36,7 @@ spmv_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ c
             const double *__restrict__ va, const double *__restrict__ x,
             double *__restrict__ y) {
     __shared__ double prod[kSpmvCap];
+    chain_begin();
     const int r0 = blockIdx.x * kSpmvRows;
     const int r1 = min(r0 + kSpmvRows, n);
     const int p0 = rp[r0], p1 = rp[r1];
@@ -45,11 +49,35 @@ spmv_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ c
         if (threadIdx.x == 0 && head && cnt > 0) prod[0] = va[p0] * __ldg(x + ci[p0]);
         const double2 *va2 = reinterpret_cast<const double2 *>(va + p0 + head);
         const int2 *ci2 = reinterpret_cast<const int2 *>(ci + p0 + head);
-        for (int t = threadIdx.x; t < npair; t += blockDim.x) {
-            const double2 v = va2[t];
-            const int2 c = ci2[t];
-            prod[head + 2 * t] = v.x * __ldg(x + c.x);
-            prod[head + 2 * t + 1] = v.y * __ldg(x + c.y);
+        // four pairs a step: the matrix's loads and then the eight gathers of
+        // x are in flight together
+        for (int t0 = threadIdx.x; t0 < npair; t0 += 4 * kSpmvRows) {
+            double2 v[4];
+            int2 c[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int t = t0 + u * kSpmvRows;
+                c[u] = make_int2(-1, -1);
+                if (t < npair) {
+                    v[u] = va2[t];
+                    c[u] = ci2[t];
+                }
+            }
+            double xa[4], xb[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (c[u].x >= 0) {
+                    xa[u] = __ldg(x + c[u].x);
+                    xb[u] = __ldg(x + c[u].y);
+                }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int t = t0 + u * kSpmvRows;
+                if (t < npair) {
+                    prod[head + 2 * t] = v[u].x * xa[u];
+                    prod[head + 2 * t + 1] = v[u].y * xb[u];
+                }
+            }
         }
         const int last = head + 2 * npair;
         if (threadIdx.x == 0 && last < cnt) prod[last] = va[p0 + last] * __ldg(x + ci[p0 + last]);
@@ -76,14 +104,14 @@ void launch_spmv(int n, const int32_t *rowptr, const int32_t *col, const double 
                  const double *x, double *y, cudaStream_t st) {
     if (n <= 0) return;
     int nb = (n + kSpmvRows - 1) / kSpmvRows;
-    spmv_kernel<<<nb, kSpmvRows, 0, st>>>(n, rowptr, col, val, x, y);
-    note_launch();
+    launch_chained(spmv_kernel, nb, kSpmvRows, 0, st, n, rowptr, col, val, x, y);
 }
 
 // ---------------------------------------------------------- tall-skinny --
 constexpr int kTsThreads = 256;
 constexpr int kTsRows = 2;       // rows per thread
-constexpr int kTsChunk = 8;      // columns reduced per register chunk
+constexpr int kTsChunk = 8;      // vectors per register chunk
+constexpr int kTsMaxBlocks = 4 * 148;
 
 static int ts_blocks(int n) {
     int nb = (n + kTsThreads * kTsRows - 1) / (kTsThreads * kTsRows);
@@ -106,10 +134,12 @@ struct TsParams {
 };
 
 // Final cross-block reduction by the last block to arrive: column c of the
-// partials is summed over blocks in a fixed order, so results are
-// reproducible run to run.
-__device__ void last_block_reduce(double *part, unsigned *counter, int ncols, double *out,
-                                  double *hcol, int hmode, double *sh) {
+// partials (nb values in a row for each column) is summed by one warp in a
+// fixed order, so results are reproducible run to run.  A chain of one L2
+// latency and the shuffles; with 512 partial sums added up by one thread the
+// reduction of a single column took 5 us.
+SPX_DEV void last_block_reduce(double *part, unsigned *counter, int ncols, double *out,
+                               double *hcol, int hmode) {
     __shared__ bool am_last;
     __threadfence();
     __syncthreads();
@@ -120,160 +150,270 @@ __device__ void last_block_reduce(double *part, unsigned *counter, int ncols, do
     __syncthreads();
     if (!am_last) return;
     __threadfence();
-    const int nb = gridDim.x;
-    const int segs = max(1, (int)blockDim.x / max(ncols, 1));
-    const int per = (nb + segs - 1) / segs;
-    // sh: ncols * segs doubles
-    for (int t = threadIdx.x; t < ncols * segs; t += blockDim.x) {
-        int c = t % ncols, s = t / ncols;
-        int b0 = s * per, b1 = min(nb, b0 + per);
-        // four independent sums keep four L2 loads in flight per thread
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int b = b0;
-        for (; b + 3 < b1; b += 4) {
-            a0 += __ldcg(part + (size_t)b * ncols + c);
-            a1 += __ldcg(part + (size_t)(b + 1) * ncols + c);
-            a2 += __ldcg(part + (size_t)(b + 2) * ncols + c);
-            a3 += __ldcg(part + (size_t)(b + 3) * ncols + c);
-        }
-        for (; b < b1; b++) a0 += __ldcg(part + (size_t)b * ncols + c);
-        sh[s * ncols + c] = (a0 + a1) + (a2 + a3);
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
+    const int nb = gridDim.x, lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < ncols; c += blockDim.x >> 5) {
+        const double *q = part + (size_t)c * nb;
         double acc = 0.0;
-        for (int s = 0; s < segs; s++) acc += sh[s * ncols + c];
-        out[c] = acc;
-        if (hmode == 1) hcol[c] = acc;
-        else if (hmode == 2) hcol[c] += acc;
+        for (int b0 = lane; b0 < nb; b0 += 32 * 10) {
+            double x[10];
+#pragma unroll
+            for (int u = 0; u < 10; u++) x[u] = b0 + 32 * u < nb ? __ldcg(q + b0 + 32 * u) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 10; u++) acc += x[u];
+        }
+        const double t = warp_sum(acc);
+        if (lane == 0) {
+            out[c] = t;
+            if (hmode == 1) hcol[c] = t;
+            else if (hmode == 2) hcol[c] += t;
+        }
     }
     if (threadIdx.x == 0) *counter = 0u;
 }
 
-// One launch covers every row: a block takes 512-row segments
-// blockIdx.x, blockIdx.x + gridDim.x, ... (the grid is capped at a few
-// blocks per SM), reduces each segment's column sums eight at a time and
-// keeps the block's running sums in shared memory; the last block to
-// finish combines the blocks' sums.
-template <int MODE>
-__global__ void __launch_bounds__(kTsThreads) ts_kernel(TsParams p) {
-    extern __shared__ double sh[];
-    const int n = p.n, m = p.m;
-    const int ncols = (MODE == TS_DOT || MODE == TS_UPDATE_DOT) ? m : 1;
-    double *hs = sh;                                  // m coefficients
-    double *bacc = hs + ((m + 1) & ~1);               // the block's column sums
-    double *red = bacc + ((ncols + 1) & ~1);          // block reduce scratch (64)
-    double *fin = red + 64;                           // last-block scratch
-    if (MODE == TS_UPDATE_DOT || MODE == TS_UPDATE_NORM)
-        for (int c = threadIdx.x; c < m; c += blockDim.x) hs[c] = p.hin[c];
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) bacc[c] = 0.0;
-    __syncthreads();
-    constexpr int kSeg = kTsThreads * kTsRows;
-    for (int64_t seg = blockIdx.x; seg * kSeg < n; seg += gridDim.x) {
-        const int64_t base = seg * kSeg + threadIdx.x;
-        double wv[kTsRows];
+// A block takes a contiguous range of rows (at most two blocks an SM, at least
+// 512 rows), in segments of kGsSeg rows of w that it keeps in shared memory:
+//   * the update w -= V h gives a thread two adjacent rows and eight columns'
+//     loads at a time; when the segment has fewer pairs of rows than half the
+//     threads, groups of threads split the columns;
+//   * the dot products give a warp one column of a share of the segment, so
+//     that no barrier stands between the loads of V: the lanes' sums are added
+//     once a column and share, into a slot of its own (a fixed order, so the
+//     result is reproducible).
+// VEC: V and w are 16-byte aligned and ldv is even, so a pair is one load.
+//
+// Bound by reading V (once a launch; the dot products after an update find
+// their segment in L2), for small n by launch, two dependent passes and the
+// reduction over blocks.  With a barrier for every eight columns of 512 rows:
+// 100^3 rows and 14 columns on average, dot 33.8, update and dot 30.9, update
+// and norm 35.7 us; 46^3 rows 11.2, 8.7, 8.3.  Now 20.2,
+// 30.3, 17.3 and 7.7, 8.9, 6.2.
+constexpr int kGsThreads = 512;
+constexpr int kGsWarps = kGsThreads / 32;
+constexpr int kGsSeg = 4096;
+constexpr int kGsMaxBlocks = 2 * 148;
+
+template <bool VEC>
+__device__ __forceinline__ double2 ts_ld2(const double *q, bool both) {
+    if (!both) return make_double2(*q, 0.0);
+    if (VEC) return *reinterpret_cast<const double2 *>(q);
+    return make_double2(q[0], q[1]);
+}
+
+// sum over c in [c0, c1) of V(i, c) h[c] for the pair of rows at v
+template <bool VEC>
+__device__ __forceinline__ double2 ts_cols(const double *v, int64_t ldv, const double *hs, int c0,
+                                           int c1, bool both) {
+    double2 s = make_double2(0.0, 0.0);
+    v += (size_t)c0 * ldv;
+    int c = c0;
+    for (; c + 8 <= c1; c += 8) {
+        double2 x[8];
 #pragma unroll
-        for (int r = 0; r < kTsRows; r++) {
-            const int64_t i = base + r * kTsThreads;
-            wv[r] = (i < n) ? p.w[i] : 0.0;
+        for (int q = 0; q < 8; q++, v += ldv) x[q] = ts_ld2<VEC>(v, both);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            s.x += x[q].x * hs[c + q];
+            s.y += x[q].y * hs[c + q];
         }
-        if (MODE == TS_UPDATE_DOT || MODE == TS_UPDATE_NORM) {
-            double s[kTsRows];
+    }
+    if (c + 4 <= c1) {
+        double2 x[4];
 #pragma unroll
-            for (int r = 0; r < kTsRows; r++) s[r] = 0.0;
-            for (int c = 0; c < m; c++) {
-                const double hc = hs[c];
-                const double *vc = p.V + (size_t)c * p.ldv;
+        for (int q = 0; q < 4; q++, v += ldv) x[q] = ts_ld2<VEC>(v, both);
 #pragma unroll
-                for (int r = 0; r < kTsRows; r++) {
-                    const int64_t i = base + r * kTsThreads;
-                    if (i < n) s[r] += vc[i] * hc;
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < kTsRows; r++) {
-                const int64_t i = base + r * kTsThreads;
-                if (i < n) { wv[r] -= s[r]; p.w[i] = wv[r]; }
-            }
+        for (int q = 0; q < 4; q++) {
+            s.x += x[q].x * hs[c + q];
+            s.y += x[q].y * hs[c + q];
         }
-        if (MODE == TS_DOT || MODE == TS_UPDATE_DOT) {
-            for (int c0 = 0; c0 < m; c0 += kTsChunk) {
-                double acc[kTsChunk];
+        c += 4;
+    }
+    if (c < c1) {
+        double2 x[3];
 #pragma unroll
-                for (int q = 0; q < kTsChunk; q++) acc[q] = 0.0;
+        for (int q = 0; q < 3; q++, v += ldv)
+            x[q] = c + q < c1 ? ts_ld2<VEC>(v, both) : make_double2(0.0, 0.0);
 #pragma unroll
-                for (int q = 0; q < kTsChunk; q++) {
-                    if (c0 + q < m) {
-                        const double *vc = p.V + (size_t)(c0 + q) * p.ldv;
-#pragma unroll
-                        for (int r = 0; r < kTsRows; r++) {
-                            const int64_t i = base + r * kTsThreads;
-                            if (i < n) acc[q] += vc[i] * wv[r];
-                        }
-                    }
-                }
-                const double t = block_sum8(acc, red);
-                if (threadIdx.x < kTsChunk && c0 + (int)threadIdx.x < m) bacc[c0 + threadIdx.x] += t;
+        for (int q = 0; q < 3; q++)
+            if (c + q < c1) {
+                s.x += x[q].x * hs[c + q];
+                s.y += x[q].y * hs[c + q];
+            }
+    }
+    return s;
+}
+
+// shares of a segment's rows for the dot products: enough items for the
+// warps, at least 256 rows an item
+__host__ __device__ inline int ts_shares(int m, int per) {
+    const int q = (per < kGsSeg ? per : kGsSeg) / 256;
+    return m > 64 ? 1 : (q < 1 ? 1 : (q > 4 ? 4 : q));
+}
+
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(kGsThreads, 2) ts_kernel(TsParams p, int per) {
+    extern __shared__ double2 ts_sm[];
+    constexpr bool UPD = MODE == TS_UPDATE_DOT || MODE == TS_UPDATE_NORM;
+    constexpr bool DOT = MODE == TS_DOT || MODE == TS_UPDATE_DOT;
+    const int m = p.m, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ncols = DOT ? m : 1, shares = DOT ? ts_shares(m, per) : 1;
+    double *ws = reinterpret_cast<double *>(ts_sm);     // kGsSeg rows of w
+    double *hs = ws + kGsSeg;                           // m coefficients
+    double *slot = hs + ((m + 1) & ~1);                 // ncols x shares
+    __shared__ double red[32];
+    chain_begin();
+    if (UPD)
+        for (int c = tid; c < m; c += kGsThreads) hs[c] = p.hin[c];
+    if (DOT)
+        for (int c = tid; c < m * shares; c += kGsThreads) slot[c] = 0.0;
+    double sq = 0.0;
+    const int64_t lo = min((int64_t)p.n, (int64_t)blockIdx.x * per);
+    const int64_t hi = min((int64_t)p.n, lo + per);
+    for (int64_t s0 = lo; s0 < hi; s0 += kGsSeg) {
+        const int len = (int)min((int64_t)kGsSeg, hi - s0), pairs = (len + 1) >> 1;
+        const double *V = p.V + s0;
+        double *w = p.w + s0;
+        __syncthreads();                                // hs, slot; the segment before is read
+        if (!UPD) {
+            for (int t = tid; t < pairs; t += kGsThreads) {
+                const double2 x = ts_ld2<VEC>(w + 2 * t, 2 * t + 1 < len);
+                if (DOT) *reinterpret_cast<double2 *>(ws + 2 * t) = x;
+                else sq += x.x * x.x + x.y * x.y;
             }
         } else {
-            double acc = 0.0;
+            int groups = 1;                             // > 1: partial sums at ws + 1024
+            while (groups < 8 && 2 * groups * pairs <= kGsThreads) groups *= 2;
+            auto finish = [&](int t, double2 s) {
+                const bool both = 2 * t + 1 < len;
+                double2 x = ts_ld2<VEC>(w + 2 * t, both);
+                x.x -= s.x;
+                x.y -= s.y;
+                if (VEC && both) {
+                    *reinterpret_cast<double2 *>(w + 2 * t) = x;
+                } else {
+                    w[2 * t] = x.x;
+                    if (both) w[2 * t + 1] = x.y;
+                }
+                if (DOT) *reinterpret_cast<double2 *>(ws + 2 * t) = x;
+                else sq += x.x * x.x + x.y * x.y;
+            };
+            for (int k = tid; k < groups * pairs; k += kGsThreads) {
+                const int g = groups > 1 ? k / pairs : 0, t = k - g * pairs;
+                const double2 s = ts_cols<VEC>(V + 2 * t, p.ldv, hs, m * g / groups,
+                                               m * (g + 1) / groups, 2 * t + 1 < len);
+                if (groups > 1) *reinterpret_cast<double2 *>(ws + 1024 + 2 * k) = s;
+                else finish(t, s);
+            }
+            if (groups > 1) {
+                __syncthreads();
+                if (tid < pairs) {
+                    double2 s = make_double2(0.0, 0.0);
+                    for (int g = 0; g < groups; g++) {
+                        const double2 v =
+                            *reinterpret_cast<const double2 *>(ws + 1024 + 2 * (g * pairs + tid));
+                        s.x += v.x;
+                        s.y += v.y;
+                    }
+                    finish(tid, s);
+                }
+            }
+        }
+        if (DOT) {
+            __syncthreads();
+            const int part = ((len + shares - 1) / shares + 63) & ~63;
+            for (int it = warp; it < m * shares; it += kGsWarps) {
+                const int sh = it / m, c = it - sh * m;
+                const int b = min(len, (sh + 1) * part);
+                const double *v = V + (size_t)c * p.ldv;
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                int r = sh * part + 2 * lane;
+                for (; r + 64 * 7 + 1 < b; r += 512) {
+                    double2 x[8];
 #pragma unroll
-            for (int r = 0; r < kTsRows; r++) acc += wv[r] * wv[r];
-            const double t = block_sum(acc, red);
-            if (threadIdx.x == 0) bacc[0] += t;
+                    for (int q = 0; q < 8; q++) x[q] = ts_ld2<VEC>(v + r + 64 * q, true);
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const double2 y = *reinterpret_cast<const double2 *>(ws + r + 64 * q);
+                        acc[q & 3] += x[q].x * y.x;
+                        acc[q & 3] += x[q].y * y.y;
+                    }
+                }
+                for (; r < b; r += 256) {
+                    double2 x[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        x[q] = r + 64 * q < b ? ts_ld2<VEC>(v + r + 64 * q, r + 64 * q + 1 < b)
+                                              : make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (r + 64 * q < b) {
+                            const double2 y = *reinterpret_cast<const double2 *>(ws + r + 64 * q);
+                            acc[q] += x[q].x * y.x;
+                            acc[q] += x[q].y * y.y;
+                        }
+                }
+                const double t = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+                if (lane == 0) slot[it] += t;
+            }
         }
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x)
-        p.part[(size_t)blockIdx.x * ncols + c] = bacc[c];
-    last_block_reduce(p.part, p.counter, ncols, p.out, p.hcol, p.hmode, fin);
+    if (DOT) {
+        for (int c = tid; c < m; c += kGsThreads) {
+            double t = 0.0;
+            for (int sh = 0; sh < shares; sh++) t += slot[sh * m + c];
+            p.part[(size_t)c * gridDim.x + blockIdx.x] = t;
+        }
+    } else {
+        sq = block_sum(sq, red);
+        if (tid == 0) p.part[blockIdx.x] = sq;
+    }
+    last_block_reduce(p.part, p.counter, ncols, p.out, p.hcol, p.hmode);
 }
-
-static size_t ts_smem(int ncols_h, int ncols_red) {
-    int segs = std::max(1, kTsThreads / std::max(ncols_red, 1));
-    return sizeof(double) * ((size_t)((ncols_h + 1) & ~1) + (size_t)((ncols_red + 1) & ~1) + 64 +
-                             (size_t)ncols_red * segs);
-}
-
-// blocks of a tall-skinny launch: one per 512-row segment, at most four per SM
-constexpr int kTsMaxBlocks = 4 * 148;
 
 template <int MODE>
-static void ts_launch(const TsParams &p, int ncols_red, cudaStream_t st) {
-    int nb = std::min(ts_blocks(p.n), kTsMaxBlocks);
-    size_t smem = ts_smem(p.m, ncols_red);
-    ts_kernel<MODE><<<nb, kTsThreads, smem, st>>>(p);
-    note_launch();
+static void ts_launch(const TsParams &p, cudaStream_t st) {
+    const int nb = std::min(ts_blocks(p.n), kGsMaxBlocks);
+    const int per = (((p.n + nb - 1) / nb) + 1) & ~1;
+    const int slots = MODE == TS_DOT || MODE == TS_UPDATE_DOT ? p.m * ts_shares(p.m, per) : 0;
+    const size_t smem = sizeof(double) * ((size_t)kGsSeg + ((p.m + 1) & ~1) + slots);
+    const bool vec = (((uintptr_t)p.V | (uintptr_t)p.w) & 15u) == 0 && p.ldv % 2 == 0;
+    if (smem > 48 * 1024)                               // more than 1000 columns
+        cudaFuncSetAttribute(vec ? ts_kernel<MODE, true> : ts_kernel<MODE, false>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_chained(vec ? ts_kernel<MODE, true> : ts_kernel<MODE, false>, nb, kGsThreads, smem, st,
+                   p, per);
 }
 
 void launch_ts_dot(const double *V, int64_t ldv, int n, int m, const double *w, double *h,
                    double *hcol, int hmode, const ReduceScratch &rs, cudaStream_t st) {
     if (m <= 0) return;
     TsParams p{V, ldv, n, m, const_cast<double *>(w), nullptr, h, hcol, hmode, rs.part, rs.counter};
-    ts_launch<TS_DOT>(p, m, st);
+    ts_launch<TS_DOT>(p, st);
 }
 void launch_ts_update_dot(const double *V, int64_t ldv, int n, int m, double *w,
                           const double *hin, double *h, double *hcol, int hmode,
                           const ReduceScratch &rs, cudaStream_t st) {
     if (m <= 0) return;
     TsParams p{V, ldv, n, m, w, hin, h, hcol, hmode, rs.part, rs.counter};
-    ts_launch<TS_UPDATE_DOT>(p, m, st);
+    ts_launch<TS_UPDATE_DOT>(p, st);
 }
 void launch_ts_update_norm(const double *V, int64_t ldv, int n, int m, double *w,
                            const double *hin, double *nrm2, const ReduceScratch &rs,
                            cudaStream_t st) {
     TsParams p{V, ldv, n, m, w, hin, nrm2, nullptr, 0, rs.part, rs.counter};
-    if (m <= 0) ts_launch<TS_NORM>(p, 1, st);
-    else ts_launch<TS_UPDATE_NORM>(p, 1, st);
+    if (m <= 0) ts_launch<TS_NORM>(p, st);
+    else ts_launch<TS_UPDATE_NORM>(p, st);
 }
 void launch_ts_norm(int n, const double *w, double *nrm2, const ReduceScratch &rs,
                     cudaStream_t st) {
     TsParams p{nullptr, 0, n, 0, const_cast<double *>(w), nullptr, nrm2, nullptr, 0, rs.part,
                rs.counter};
-    ts_launch<TS_NORM>(p, 1, st);
+    ts_launch<TS_NORM>(p, st);
 }
 
 __global__ void scale_invnorm_kernel(int n, const double *src, const double *nrm2, double *dst) {
+    chain_begin();
     const double s = 1.0 / sqrt(nrm2[0]);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         dst[i] = src[i] * s;
@@ -281,8 +421,7 @@ __global__ void scale_invnorm_kernel(int n, const double *src, const double *nrm
 void launch_scale_by_invnorm(int n, const double *src, const double *nrm2, double *dst,
                              cudaStream_t st) {
     int nb = std::min(4096, (n + 255) / 256);
-    scale_invnorm_kernel<<<std::max(nb, 1), 256, 0, st>>>(n, src, nrm2, dst);
-    note_launch();
+    launch_chained(scale_invnorm_kernel, std::max(nb, 1), 256, 0, st, n, src, nrm2, dst);
 }
 
 // ------------------------------------------------------ Ritz / residual --
@@ -301,80 +440,107 @@ struct RitzParams {
     unsigned *counter;
 };
 
+// A thread takes two adjacent rows and eight vectors at a time, with four
+// columns' loads in flight; a block loops over 512-row segments (at most four
+// blocks an SM) and adds its squared norms up per warp, with one barrier at
+// the end.  Bound by reading V once for every eight vectors (out of L2 after
+// the first).  20 columns, 6 vectors at 100^3 rows: 120 -> 56 us (two rows of
+// separate loads, one column in flight and a barrier a vector before).
+template <bool VEC>
 __global__ void __launch_bounds__(kTsThreads) ritz_kernel(RitzParams p) {
-    extern __shared__ double sh[];
-    const int m = p.m, nv = p.nvec;
-    double *Ss = sh;                                  // m x nv
-    double *red = Ss + (((size_t)m * nv + 1) & ~1);
-    double *fin = red + 32;
-    for (int t = threadIdx.x; t < m * nv; t += blockDim.x) {
-        int c = t % m, v = t / m;
-        Ss[t] = p.S[(size_t)p.idx[p.idx_off + v] * p.lds + c];
+    extern __shared__ double2 ritz_sm[];
+    chain_begin();
+    const int m = p.m, nv = p.nvec, nvp = (nv + kTsChunk - 1) & ~(kTsChunk - 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double *Ss = reinterpret_cast<double *>(ritz_sm);  // m x nvp, a column's vectors adjacent
+    double *slot = Ss + (size_t)m * nvp;               // warps x nvp
+    for (int t = tid; t < m * nvp; t += kTsThreads) {
+        const int c = t / nvp, v = t - c * nvp;
+        Ss[t] = v < nv ? p.S[(size_t)p.idx[p.idx_off + v] * p.lds + c] : 0.0;
     }
+    for (int t = tid; t < (kTsThreads / 32) * nvp; t += kTsThreads) slot[t] = 0.0;
     __syncthreads();
-    const int base = blockIdx.x * (kTsThreads * kTsRows) + threadIdx.x;
-    for (int v0 = 0; v0 < nv; v0 += kTsChunk) {
-        double acc[kTsChunk][kTsRows];
+    constexpr int kSeg = kTsThreads * kTsRows;
+    for (int64_t base = (int64_t)blockIdx.x * kSeg; base < p.n; base += (int64_t)gridDim.x * kSeg) {
+        const int64_t i = base + 2 * tid;
+        const bool any = i < p.n, both = i + 1 < p.n;
+        const double *v0p = p.V + i;
+        for (int v0 = 0; v0 < nv; v0 += kTsChunk) {
+            double a0[kTsChunk], a1[kTsChunk];
 #pragma unroll
-        for (int q = 0; q < kTsChunk; q++)
+            for (int q = 0; q < kTsChunk; q++) a0[q] = a1[q] = 0.0;
+            if (any)
+                for (int c0 = 0; c0 < m; c0 += 4) {
+                    double2 x[4];
 #pragma unroll
-            for (int r = 0; r < kTsRows; r++) acc[q][r] = 0.0;
-        for (int c = 0; c < m; c++) {
-            const double *vc = p.V + (size_t)c * p.ldv;
-            double vr[kTsRows];
+                    for (int u = 0; u < 4; u++)
+                        if (c0 + u < m) x[u] = ts_ld2<VEC>(v0p + (size_t)(c0 + u) * p.ldv, both);
 #pragma unroll
-            for (int r = 0; r < kTsRows; r++) {
-                int i = base + r * kTsThreads;
-                vr[r] = (i < p.n) ? vc[i] : 0.0;
-            }
+                    for (int u = 0; u < 4; u++)
+                        if (c0 + u < m) {
+                            const double *s = Ss + (size_t)(c0 + u) * nvp + v0;
+#pragma unroll
+                            for (int q = 0; q < kTsChunk; q += 2) {
+                                const double2 sv = *reinterpret_cast<const double2 *>(s + q);
+                                a0[q] += x[u].x * sv.x;
+                                a1[q] += x[u].y * sv.x;
+                                a0[q + 1] += x[u].x * sv.y;
+                                a1[q + 1] += x[u].y * sv.y;
+                            }
+                        }
+                }
 #pragma unroll
             for (int q = 0; q < kTsChunk; q++) {
-                if (v0 + q < nv) {
-                    const double s = Ss[(size_t)(v0 + q) * m + c];
-#pragma unroll
-                    for (int r = 0; r < kTsRows; r++) acc[q][r] += vr[r] * s;
+                if (v0 + q >= nv) break;
+                if (any) {
+                    double *x = p.X + (size_t)(v0 + q) * p.ldx + i;
+                    if (VEC && both) {
+                        *reinterpret_cast<double2 *>(x) = make_double2(a0[q], a1[q]);
+                    } else {
+                        x[0] = a0[q];
+                        if (both) x[1] = a1[q];
+                    }
                 }
+                double t = any ? a0[q] * a0[q] : 0.0;
+                if (both) t += a1[q] * a1[q];
+                t = warp_sum(t);
+                if (lane == 0) slot[warp * nvp + v0 + q] += t;
             }
-        }
-#pragma unroll
-        for (int q = 0; q < kTsChunk; q++) {
-            if (v0 + q >= nv) continue;
-            double sq = 0.0;
-#pragma unroll
-            for (int r = 0; r < kTsRows; r++) {
-                int i = base + r * kTsThreads;
-                if (i < p.n) {
-                    p.X[(size_t)(v0 + q) * p.ldx + i] = acc[q][r];
-                    sq += acc[q][r] * acc[q][r];
-                }
-            }
-            double t = block_sum(sq, red);
-            if (threadIdx.x == 0) p.part[(size_t)blockIdx.x * nv + v0 + q] = t;
         }
     }
-    last_block_reduce(p.part, p.counter, nv, p.nrm2, nullptr, 0, fin);
+    __syncthreads();
+    for (int v = tid; v < nv; v += kTsThreads) {
+        double t = 0.0;
+        for (int q = 0; q < kTsThreads / 32; q++) t += slot[q * nvp + v];
+        p.part[(size_t)v * gridDim.x + blockIdx.x] = t;
+    }
+    last_block_reduce(p.part, p.counter, nv, p.nrm2, nullptr, 0);
 }
 
 void launch_ritz_vectors(const double *V, int64_t ldv, int n, int m, const double *S, int lds,
                          const int *idx, int idx_off, int nvec, double *X, int64_t ldx,
                          double *nrm2, const ReduceScratch &rs, cudaStream_t st) {
     if (nvec <= 0) return;
-    // vectors per launch: the m x nv block of S fits the default 48 KB of
-    // dynamic shared memory beside the reduction scratch
-    const int cap = std::max(1, (6144 - 32 - 2 * kTsThreads) / std::max(1, m));
+    // vectors per launch: the m x nv block of S and the warps' sums fit 48 KB
+    // of shared memory, but at least one chunk of eight (opting in to more
+    // where m is above 760)
+    const int cap = std::max(kTsChunk, 6144 / (m + 8) / kTsChunk * kTsChunk);
+    const bool vec = (((uintptr_t)V | (uintptr_t)X) & 15u) == 0 && ldv % 2 == 0 && ldx % 2 == 0;
     for (int v0 = 0; v0 < nvec; v0 += cap) {
-        const int nv = std::min(cap, nvec - v0);
+        const int nv = std::min(cap, nvec - v0), nvp = (nv + kTsChunk - 1) & ~(kTsChunk - 1);
         RitzParams p{V, ldv, n, m, S, lds, idx, idx_off + v0, nv, X + (size_t)v0 * ldx, ldx,
                      nrm2 + v0, rs.part, rs.counter};
-        int nb = ts_blocks(n);
-        int segs = std::max(1, kTsThreads / nv);
-        size_t smem = sizeof(double) * ((((size_t)m * nv + 1) & ~1) + 32 + (size_t)nv * segs);
-        ritz_kernel<<<nb, kTsThreads, smem, st>>>(p);
-        note_launch();
+        const int nb = std::min(ts_blocks(n), kTsMaxBlocks);
+        const size_t smem = sizeof(double) * (size_t)(m + kTsThreads / 32) * nvp;
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(vec ? ritz_kernel<true> : ritz_kernel<false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_chained(vec ? ritz_kernel<true> : ritz_kernel<false>, nb, kTsThreads, smem, st, p);
     }
 }
 
 __global__ void scale_cols_kernel(int n, int nvec, double *X, int64_t ldx, const double *nrm2) {
+    chain_begin();
     const int v = blockIdx.y;
     const double q = nrm2[v];
     if (!(q > 0.0)) return;
@@ -387,8 +553,7 @@ void launch_scale_cols(int n, int nvec, double *X, int64_t ldx, const double *nr
                        cudaStream_t st) {
     if (nvec <= 0) return;
     int nb = std::max(1, std::min(1024, (n + 255) / 256));
-    scale_cols_kernel<<<dim3(nb, nvec), 256, 0, st>>>(n, nvec, X, ldx, nrm2);
-    note_launch();
+    launch_chained(scale_cols_kernel, dim3(nb, nvec), 256, 0, st, n, nvec, X, ldx, nrm2);
 }
 
 struct RqParams {
@@ -403,39 +568,61 @@ struct RqParams {
     unsigned *counter;
 };
 
+// Four rows a thread and vector in flight, blocks over all rows (at most four
+// an SM), one barrier at the end.  Bound by reading X and AX.  6 vectors of
+// 100^3 rows: 37 -> 21 us a pass (a barrier for every vector of 512 rows
+// before).
 __global__ void __launch_bounds__(kTsThreads) rq_kernel(RqParams p) {
     extern __shared__ double sh[];
-    double *red = sh, *fin = sh + 32;
-    const int base = blockIdx.x * (kTsThreads * kTsRows) + threadIdx.x;
+    constexpr int kWarps = kTsThreads / 32;
+    double *slot = sh;
+    chain_begin();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * kTsThreads;
     for (int v = 0; v < p.nvec; v++) {
         const double *x = p.X + (size_t)v * p.ldx, *ax = p.AX + (size_t)v * p.ldax;
         const double lam = (p.pass == 1) ? p.lam[v] : 0.0;
         double acc = 0.0;
+        for (int64_t i0 = (int64_t)blockIdx.x * kTsThreads + threadIdx.x; i0 < p.n; i0 += 4 * step) {
+            double a[4], b[4];
 #pragma unroll
-        for (int r = 0; r < kTsRows; r++) {
-            int i = base + r * kTsThreads;
-            if (i < p.n) {
-                if (p.pass == 0) acc += x[i] * ax[i];
-                else { double d = ax[i] - lam * x[i]; acc += d * d; }
+            for (int r = 0; r < 4; r++) {
+                const int64_t i = i0 + r * step;
+                a[r] = i < p.n ? x[i] : 0.0;
+                b[r] = i < p.n ? ax[i] : 0.0;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                if (i0 + r * step >= p.n) break;
+                if (p.pass == 0) acc += a[r] * b[r];
+                else { const double d = b[r] - lam * a[r]; acc += d * d; }
             }
         }
-        double t = block_sum(acc, red);
-        if (threadIdx.x == 0) p.part[(size_t)blockIdx.x * p.nvec + v] = t;
+        acc = warp_sum(acc);
+        if (lane == 0) slot[v * kWarps + warp] = acc;
     }
-    last_block_reduce(p.part, p.counter, p.nvec, p.pass == 0 ? p.lam : p.r2, nullptr, 0, fin);
+    __syncthreads();
+    for (int v = threadIdx.x; v < p.nvec; v += kTsThreads) {
+        double t = 0.0;
+        for (int q = 0; q < kWarps; q++) t += slot[v * kWarps + q];
+        p.part[(size_t)v * gridDim.x + blockIdx.x] = t;
+    }
+    last_block_reduce(p.part, p.counter, p.nvec, p.pass == 0 ? p.lam : p.r2, nullptr, 0);
 }
 
 void launch_rayleigh_resid(int n, int nvec, const double *X, int64_t ldx, const double *AX,
                            int64_t ldax, double *lam, double *r2, const ReduceScratch &rs,
                            cudaStream_t st) {
-    if (nvec <= 0) return;
-    int nb = ts_blocks(n);
-    int segs = std::max(1, kTsThreads / nvec);
-    size_t smem = sizeof(double) * (32 + (size_t)nvec * segs);
-    for (int pass = 0; pass < 2; pass++) {
-        RqParams p{n, nvec, X, ldx, AX, ldax, lam, r2, pass, rs.part, rs.counter};
-        rq_kernel<<<nb, kTsThreads, smem, st>>>(p);
-        note_launch();
+    const int cap = 512;                 // vectors per launch: 32 KB of warps' sums
+    for (int v0 = 0; v0 < nvec; v0 += cap) {
+        const int nv = std::min(cap, nvec - v0);
+        const int nb = std::min(ts_blocks(n), kTsMaxBlocks);
+        const size_t smem = sizeof(double) * (size_t)nv * (kTsThreads / 32);
+        for (int pass = 0; pass < 2; pass++) {
+            RqParams p{n, nv, X + (size_t)v0 * ldx, ldx, AX + (size_t)v0 * ldax, ldax, lam + v0,
+                       r2 + v0, pass, rs.part, rs.counter};
+            launch_chained(rq_kernel, nb, kTsThreads, smem, st, p);
+        }
     }
 }
 
@@ -832,22 +1019,22 @@ void launch_set_diag(int ldh, int nd, const double *d, double *H, cudaStream_t s
 }
 
 __global__ void flag_if_below_kernel(const double *nrm2, double thr, int *flag) {
+    chain_begin();
     if (!(nrm2[0] >= thr)) *flag = 1;
 }
 void launch_flag_if_below(const double *nrm2, double thr, int *flag, cudaStream_t st) {
-    flag_if_below_kernel<<<1, 1, 0, st>>>(nrm2, thr, flag);
-    note_launch();
+    launch_chained(flag_if_below_kernel, 1, 1, 0, st, nrm2, thr, flag);
 }
 
 __global__ void set_beta_kernel(double *H, int ldh, int r, int c, const double *nrm2, int zero) {
+    chain_begin();
     double b = zero ? 0.0 : sqrt(nrm2[0]);
     H[r + (size_t)c * ldh] = b;
     H[c + (size_t)r * ldh] = b;
 }
 void launch_set_beta(double *H, int ldh, int r, int c, const double *nrm2, int zero,
                      cudaStream_t st) {
-    set_beta_kernel<<<1, 1, 0, st>>>(H, ldh, r, c, nrm2, zero);
-    note_launch();
+    launch_chained(set_beta_kernel, 1, 1, 0, st, H, ldh, r, c, nrm2, zero);
 }
 
 __global__ void copy_kernel(int64_t n, const double *src, double *dst) {

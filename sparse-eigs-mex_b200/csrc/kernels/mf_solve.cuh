@@ -649,6 +649,7 @@ template <int NR>
 __global__ void __launch_bounds__(SShared<NR>::kThreads, NR == 1 ? 8 : NR == 8 ? 3 : 2) mf_solve(SolveArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SShared<NR> &sh = *reinterpret_cast<SShared<NR> *>(smem_raw);
+    chain_begin();
     if (a.skip && *(volatile const int *)a.skip) return;
     const int tid = threadIdx.x;
     if (tid == 0) {

@@ -7,6 +7,7 @@
 // pivot that is not positive records the failing column in a device status
 // word (never a trap); the tasks after it do no work.
 #include "multifrontal.cuh"
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 #include "../host/parallel.h"
@@ -798,12 +799,11 @@ template <> int MultifrontalPlanT<Real>::run_solve(int q, const double *B, int64
     a.accumulate = accumulate ? 1 : 0;
     a.skip = skip;
     const int grid = std::min(sgrid_[q], a.ntasks);
-    if (q == 0) mf_solve<1><<<grid, kVecThreads, sizeof(SShared<1>), st>>>(a);
-    else if (q == 1) mf_solve<8><<<grid, kBlkThreads, sizeof(SShared<8>), st>>>(a);
-    else if (q == 2) mf_solve<16><<<grid, kBlkThreads, sizeof(SShared<16>), st>>>(a);
-    else if (q == 3) mf_solve<24><<<grid, kBlkThreads, sizeof(SShared<24>), st>>>(a);
-    else mf_solve<32><<<grid, kBlkThreads, sizeof(SShared<32>), st>>>(a);
-    note_launch();
+    if (q == 0) launch_chained(mf_solve<1>, grid, kVecThreads, sizeof(SShared<1>), st, a);
+    else if (q == 1) launch_chained(mf_solve<8>, grid, kBlkThreads, sizeof(SShared<8>), st, a);
+    else if (q == 2) launch_chained(mf_solve<16>, grid, kBlkThreads, sizeof(SShared<16>), st, a);
+    else if (q == 3) launch_chained(mf_solve<24>, grid, kBlkThreads, sizeof(SShared<24>), st, a);
+    else launch_chained(mf_solve<32>, grid, kBlkThreads, sizeof(SShared<32>), st, a);
     return 0;
 }
 

@@ -2,6 +2,7 @@
 // block per component, every vector operation of the reference's lanczos()
 // (src/speigs_core.c:146-315) restricted to the component's row segment.
 #include "seg_lanczos.cuh"
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(kSegThreads) seg_start_kernel(SegArgs a, uint6
 __global__ void __launch_bounds__(kSegThreads) seg_step_kernel(SegArgs a) {
     extern __shared__ double sh[];
     __shared__ uint64_t s_seed;
+    chain_begin();
     const int c = blockIdx.x;
     if (!a.ext[c]) return;
     const SegSmem sm = seg_smem(sh, a.ncv);
@@ -333,8 +335,7 @@ void launch_seg_start(const SegArgs &a, uint64_t seed, cudaStream_t st) {
     note_launch();
 }
 void launch_seg_step(const SegArgs &a, cudaStream_t st) {
-    seg_step_kernel<<<a.nseg, kSegThreads, seg_smem_bytes(a.ncv), st>>>(a);
-    note_launch();
+    launch_chained(seg_step_kernel, a.nseg, kSegThreads, seg_smem_bytes(a.ncv), st, a);
 }
 void launch_seg_ritz(const SegArgs &a, cudaStream_t st) {
     seg_ritz_kernel<<<a.nseg, kSegThreads, seg_smem_bytes(a.ncv), st>>>(a);
