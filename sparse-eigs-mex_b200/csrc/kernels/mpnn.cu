@@ -12,6 +12,7 @@
 // onto span(Y) and U the k eigenvectors the solver computed for the same
 // operator; its gradient is dL/dY = -(2/k) (U - Y C) C^T with
 // C = (Y^T Y)^{-1} Y^T U.  Adam updates the FP32 weights.
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 #include "../../../include/speigs_b200.h"
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(kThreads)
 spmm_add_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                 const float *__restrict__ w, const float *__restrict__ in, float *__restrict__ out) {
     const int lane = threadIdx.x & 31, f = lane & 15, g0 = lane & 16;
+    spx::chain_begin();
     const int row = blockIdx.x * (kThreads / 16) + (threadIdx.x >> 4);
     int q = row < n ? rp[row] : 0;
     const int q1 = row < n ? rp[row + 1] : 0;
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(kThreads)
 input_fwd_kernel(int n, int F, const float *__restrict__ X, const bf16 *__restrict__ W,
                  const float *__restrict__ b, bf16 *__restrict__ out) {
     extern __shared__ float4 in_sm[];
+    spx::chain_begin();
     float *Ws = reinterpret_cast<float *>(in_sm);   // F x 64: W transposed
     float *Xs = Ws + F * kHid;                      // kInRows x (F + 1)
     const int r0 = blockIdx.x * kInRows;
@@ -220,6 +223,7 @@ dense_bwd_kernel(int n, int F, const TX *__restrict__ X1, const bf16 *__restrict
     constexpr int CG = K / 8;               // thread columns: 4 cg + {0..3} and K / 2 + the same
     constexpr int TR = kRows * CG / kThreads;   // thread rows
     extern __shared__ float4 bwd_sm[];
+    spx::chain_begin();
     float *Ws = reinterpret_cast<float *>(bwd_sm);   // 64 x K, rows >= N zero
     float *Xs = Ws + kHid * K;                       // kRows x K
     float *Zs = Xs + kRows * K;                      // kRows x kZs, columns >= N zero
@@ -386,7 +390,7 @@ dense_bwd_kernel(int n, int F, const TX *__restrict__ X1, const bf16 *__restrict
 // at 48^3), then tanhf.  The messages and, where the caller does not train,
 // the last activations never go to memory.  48^3 nodes: 27 us a layer
 // against 29 for the messages and 32 for the dense part in launches of their
-// own; the whole forward pass 305 -> 124 us.  Three blocks fit an SM (56 KB
+// own; the whole forward pass 301 -> 115 us.  Three blocks fit an SM (56 KB
 // of shared memory each), enough for 24 warps of gathers while one block is
 // in its epilogue.
 constexpr int kTcRows = 128;
@@ -475,6 +479,7 @@ layer_fwd_kernel(int n, const int32_t *__restrict__ rp, const int32_t *__restric
                  int P, const bf16 *__restrict__ Wo, const float *__restrict__ bo,
                  float *__restrict__ Y, volatile int *err) {
     extern __shared__ unsigned char tc_sm[];
+    spx::chain_begin();
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ float s_b[kHid], s_bo[kHid];
@@ -689,6 +694,7 @@ __global__ void __launch_bounds__(kThreads)
 gram_kernel(int n, int P, const float *__restrict__ Y, int k, const float *__restrict__ U,
             double *G, double *B) {
     extern __shared__ double2 gram_sm[];
+    spx::chain_begin();
     double *S = reinterpret_cast<double *>(gram_sm);    // kGramRows x ld: [Y, U, 0]
     const int Q = P + k, ld = (Q + 1) & ~1;
     const int64_t r0 = (int64_t)blockIdx.x * kGramRows;
@@ -733,6 +739,7 @@ __global__ void __launch_bounds__(kSolveThreads)
 small_solve_kernel(int P, int k, const double *__restrict__ G, const double *__restrict__ B,
                    float *__restrict__ C, double *loss) {
     constexpr int LD = 65;
+    spx::chain_begin();
     __shared__ double L[64 * LD], s_inv[64];
     __shared__ double s_tr;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -800,6 +807,7 @@ __global__ void __launch_bounds__(kThreads)
 dy_kernel(int n, int P, int k, const float *__restrict__ Y, const float *__restrict__ U,
           const float *__restrict__ C, float *__restrict__ dY) {
     extern __shared__ float dy_sm[];
+    spx::chain_begin();
     const int lp = P | 1, lk = k | 1;
     float *Cs = dy_sm, *Ys = Cs + P * lk, *Es = Ys + kRows * lp;
     const int64_t r0 = (int64_t)blockIdx.x * kRows;
@@ -948,9 +956,9 @@ float *forward(speigs_mpnn_s *net, int n, const int32_t *rp, const int32_t *ci, 
     float *Y = tco && !keep && aligned16(Yout) ? Yout : net->Y;
     const bf16 *Wo = net->pb + net->woff[L + 1];
     const float *bo = net->p + net->boff[L + 1];
-    input_fwd_kernel<<<(n + kInRows - 1) / kInRows, kThreads, input_smem(net->F), st>>>(
-        n, net->F, X, net->pb + net->woff[0], net->p + net->boff[0], net->Hs);
-    spx::note_launch();
+    spx::launch_chained(input_fwd_kernel, (n + kInRows - 1) / kInRows, kThreads,
+                        input_smem(net->F), st, n, net->F, X, net->pb + net->woff[0], net->p +
+                        net->boff[0], net->Hs);
     for (int l = 1; l <= L; l++) {
         bf16 *Hp = net->Hs + (size_t)(l - 1) * n * H, *Hn = net->Hs + (size_t)l * n * H;
         bf16 *Ml = net->Ms + (size_t)(l - 1) * n * H;
@@ -958,10 +966,9 @@ float *forward(speigs_mpnn_s *net, int n, const int32_t *rp, const int32_t *ci, 
         const float *b = net->p + net->boff[l];
         if (tc) {
             const bool last = l == L && tco;
-            layer_fwd_kernel<<<tb, kTcThreads, kTcSmem, st>>>(
-                n, rp, ci, w, Hp, keep ? Ml : nullptr, W, b, last && !keep ? nullptr : Hn, P, Wo,
-                bo, last ? Y : nullptr, net->err_d);
-            spx::note_launch();
+            spx::launch_chained(layer_fwd_kernel, tb, kTcThreads, kTcSmem, st, n, rp, ci, w, Hp,
+                                keep ? Ml : nullptr, W, b, last && !keep ? nullptr : Hn, P, Wo, bo,
+                                last ? Y : nullptr, net->err_d);
         } else {
             spmm_kernel<<<(n + 7) / 8, 256, 0, st>>>(n, H, rp, ci, w, Hp, Ml);
             dense_fwd_kernel<bf16><<<nb, kThreads, dense_smem(2 * H, H), st>>>(n, H, Hp, H, Ml, H,
@@ -974,10 +981,10 @@ float *forward(speigs_mpnn_s *net, int n, const int32_t *rp, const int32_t *ci, 
         dense_fwd_kernel<float><<<nb, kThreads, dense_smem(H, P), st>>>(n, H, HL, 0, nullptr, P, Wo,
                                                                         bo, 0, Y);
     else if (L == 0)
-        layer_fwd_kernel<<<tb, kTcThreads, kTcSmem, st>>>(n, nullptr, nullptr, nullptr, HL, nullptr,
-                                                          nullptr, nullptr, nullptr, P, Wo, bo, Y,
-                                                          net->err_d);
-    if (!tco || L == 0) spx::note_launch();
+        spx::launch_chained(layer_fwd_kernel, tb, kTcThreads, kTcSmem, st, n, nullptr, nullptr,
+                            nullptr, HL, nullptr, nullptr, nullptr, nullptr, P, Wo, bo, Y,
+                            net->err_d);
+    if (!tco) spx::note_launch();
     return Y;
 }
 
@@ -1137,33 +1144,33 @@ int speigs_b200_mpnn_train_step(speigs_mpnn net, int64_t n, const int32_t *rowpt
     // loss and dL/dY
     double *G = net->G, *B = G + (size_t)P * P;
     cudaMemsetAsync(G, 0, sizeof(double) * (size_t)P * (P + k), st);
-    gram_kernel<<<(nn + kGramRows - 1) / kGramRows, kThreads,
-                  sizeof(double) * kGramRows * ((P + k + 1) & ~1), st>>>(nn, P, net->Y, k, U, G, B);
-    small_solve_kernel<<<1, kSolveThreads, 0, st>>>(P, k, G, B, net->C, net->loss);
-    dy_kernel<<<nb, kThreads, dy_smem(P, k), st>>>(nn, P, k, net->Y, U, net->C, net->dY);
-    spx::note_launch(3);
+    spx::launch_chained(gram_kernel, (nn + kGramRows - 1) / kGramRows, kThreads, sizeof(double) *
+                        kGramRows * ((P + k + 1) & ~1), st, nn, P, net->Y, k, U, G, B);
+    spx::launch_chained(small_solve_kernel, 1, kSolveThreads, 0, st, P, k, G, B, net->C,
+                        net->loss);
+    spx::launch_chained(dy_kernel, nb, kThreads, dy_smem(P, k), st, nn, P, k, net->Y, U, net->C,
+                        net->dY);
     // backward
     cudaMemsetAsync(net->g, 0, sizeof(float) * net->nparam, st);
-    dense_bwd_kernel<64, bf16><<<bb, kThreads, bwd_smem<64>(), st>>>(
-        nn, H, net->Hs + (size_t)L * nn * H, nullptr, P, net->pb + net->woff[L + 1], nullptr,
-        net->dY, net->dH, nullptr, net->g + net->woff[L + 1], net->g + net->boff[L + 1]);
-    spx::note_launch();
+    spx::launch_chained(dense_bwd_kernel<64, bf16>, bb, kThreads, bwd_smem<64>(), st, nn, H,
+                        net->Hs + (size_t)L * nn * H, nullptr, P, net->pb + net->woff[L + 1],
+                        nullptr, net->dY, net->dH, nullptr, net->g + net->woff[L + 1], net->g +
+                        net->boff[L + 1]);
     for (int l = L; l >= 1; l--) {
         bf16 *Hp = net->Hs + (size_t)(l - 1) * nn * H, *Hn = net->Hs + (size_t)l * nn * H;
         bf16 *Ml = net->Ms + (size_t)(l - 1) * nn * H;
         // dH holds dL/dh_l; produce dL/dh_{l-1} (direct part) and dL/dm_l
-        dense_bwd_kernel<128, bf16><<<bb, kThreads, bwd_smem<128>(), st>>>(
-            nn, 2 * H, Hp, Ml, H, net->pb + net->woff[l], Hn, net->dH, net->dH2, net->dM,
-            net->g + net->woff[l], net->g + net->boff[l]);
+        spx::launch_chained(dense_bwd_kernel<128, bf16>, bb, kThreads, bwd_smem<128>(), st, nn, 2 *
+                            H, Hp, Ml, H, net->pb + net->woff[l], Hn, net->dH, net->dH2, net->dM,
+                            net->g + net->woff[l], net->g + net->boff[l]);
         // dL/dh_{l-1} = direct part + A^T dL/dm_l (A symmetric)
-        spmm_add_kernel<<<sb, kThreads, 0, st>>>(nn, rowptr, col, w, net->dM, net->dH2);
+        spx::launch_chained(spmm_add_kernel, sb, kThreads, 0, st, nn, rowptr, col, w, net->dM,
+                            net->dH2);
         std::swap(net->dH, net->dH2);
-        spx::note_launch(2);
     }
-    dense_bwd_kernel<64, float><<<bb, kThreads, bwd_smem<64>(), st>>>(
-        nn, net->F, X, nullptr, H, net->pb + net->woff[0], net->Hs, net->dH, nullptr, nullptr,
-        net->g + net->woff[0], net->g + net->boff[0]);
-    spx::note_launch();
+    spx::launch_chained(dense_bwd_kernel<64, float>, bb, kThreads, bwd_smem<64>(), st, nn, net->F,
+                        X, nullptr, H, net->pb + net->woff[0], net->Hs, net->dH, nullptr, nullptr,
+                        net->g + net->woff[0], net->g + net->boff[0]);
     if (lr > 0.f) {
         net->step++;
         const float b1 = 0.9f, b2 = 0.999f;
