@@ -24,28 +24,28 @@
 // per row block and a backward tile a few columns of every row block, both
 // long enough for bulk copies.
 //
-// What bounds it: the tasks' latency, not bytes.  A task is a chain of a
-// dozen short waits (queue, flag, gather, barriers, flag), so throughput is
-// the number of tiles in flight: small blocks (one right-hand side: four
-// warps, eight blocks to an SM with a 16 KB tile each), and the next task's record fetched and its tile and
-// lists copied while the current one finishes.  A block takes the next task's
-// number only when the current one's probe is there: a block that waits for
-// its inputs then holds no other task back (taken at the start of the task,
-// 33x35x37 0.134 ms and 46^3 0.186; a second task further ahead, 46^3 0.215).
-// The tiles of the single
-// solve are a few rows times all columns (forward) or a few columns times
-// all rows (backward), so that most supernodes need no sum across blocks.  A
-// row (column) chunk wider (taller) than a tile is cut into strips whose
-// partial products the task of the last strip waits for and adds in a fixed
-// order, so results are the same every run.  With several right-hand sides the
-// gathers cost more than the panel, so forward tiles are 64 x 64 and backward
-// ones a few columns of 256 rows.
+// What bounds it: the tasks' latency and, with one right-hand side, the
+// instructions around their few products, not bytes.  A task is a chain of a
+// dozen short waits (queue, gather, barriers), so throughput is the number of
+// tiles in flight: small blocks (one right-hand side: four warps, eight blocks
+// to an SM with a 16 KB tile each), and the next task's record fetched and its
+// tile and lists copied while the current one finishes.  A block takes the
+// next task's number only when the current one's probe is there: a block that
+// waits for its inputs then holds no other task back (taken at the start of
+// the task, 33x35x37 0.134 ms instead of 0.094, 46^3 0.186 instead of 0.162).
+// The tiles of the single solve are a few rows times all columns (forward) or
+// a few columns times all rows (backward), so that most supernodes need no sum
+// across blocks.  A row (column) chunk wider (taller) than a tile is cut into
+// strips whose partial products the task of the last strip waits for and adds
+// in a fixed order, so results are the same every run.  With several
+// right-hand sides the gathers cost more than the panel, so forward tiles are
+// 64 x 64 and backward ones a few columns of 256 rows.
 //
 // Measured against the solve of before (flags and last-arrival counters,
 // 64 x 128 tiles, two blocks an SM) on the same supernodes: one right-hand
-// side 20^3 0.089 -> 0.061 ms, 33x35x37 0.188 -> 0.140, 46^3 0.347 -> 0.190,
-// 64^3 1.03 -> 0.50 (1.66 GB of panels, 3.3 TB/s); eight at 48^3 0.442 ->
-// 0.326, 24 at 48^3 0.80 -> 0.71.
+// side 20^3 0.089 -> 0.049 ms, 33x35x37 0.188 -> 0.082, 46^3 0.347 -> 0.148,
+// 64^3 1.03 -> 0.467 (1.66 GB of panels, 3.6 TB/s); eight at 48^3 0.442 ->
+// 0.290, 24 at 48^3 0.80 -> 0.67.
 constexpr int kVecThreads = 128, kBlkThreads = 256;
 constexpr int kVecElems = 2048;      // panel entries of a tile, NR = 1
 constexpr int kVecRows = 128;        // rows of a forward tile, NR = 1
@@ -112,7 +112,7 @@ struct SShared {
     Real panel[kElems];
     int lists[kLists];
     double vec[NR == 1 ? kVecTall * 16 : kBlkTall * 16 * SEG];
-    double part[kVecThreads];
+    double part[2 * kVecThreads];        // NR = 1
     STask task[2];
     unsigned long long lfull, pfull;     // lists, panel in place
 };
@@ -295,33 +295,41 @@ SPX_DEV void sum_strips2(double2 (&s)[NCH], const double *p0, int64_t step, int 
     }
 }
 
-// entries q0 <= q < q1 of the gather list, summed in order; four loads at a
-// time in flight
+// entries q0 <= q < q1 of the gather list, summed in order; two loads at a
+// time in flight (most rows get one or two)
 SPX_DEV double sum_vals(const SolveArgs &a, const double *u, const int *ci, int lo, bool staged,
                         int q0, int q1) {
     double s = 0.0;
-    for (int q = q0; q < q1; q += 4) {
-        const double *p[4];
-        double v[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int at = q + e;
-            p[e] = u + (at < q1 ? (staged ? ci[at - lo] : a.cidx[at]) : 0);
-            v[e] = at < q1 ? ld_val(p[e]) : 0.0;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            if (q + e < q1) s += got(v[e], p[e], a.err);
+    for (int q = q0; q < q1; q += 2) {
+        const bool two = q + 1 < q1;
+        const double *p0 = u + (staged ? ci[q - lo] : a.cidx[q]);
+        const double *p1 = two ? u + (staged ? ci[q + 1 - lo] : a.cidx[q + 1]) : p0;
+        const double v0 = ld_val(p0);
+        double v1 = 0.0;
+        if (two) v1 = ld_val(p1);
+        s += got(v0, p0, a.err);
+        if (two) s += got(v1, p1, a.err);
     }
     return s;
 }
 
 // ---- one right-hand side ------------------------------------------------
-// Thread t works on row t % 16 of its group's row blocks; the 8 groups
-// share the tile's row blocks and, where those are fewer, its columns
-// (forward); or its columns and, where those are fewer, its row blocks
-// (backward).  Either way 16 products a thread, then one small sum.
-SPX_DEV int pow2_at_least(int v) { return v <= 1 ? 1 : 1 << (32 - __clz(v - 1)); }
+// Thread t works on rows 2 (t % 8) and the next of its group's row blocks;
+// the 16 groups share the tile's row blocks and, where those are fewer, its
+// columns (forward); or its columns and, where those are fewer, its row blocks
+// (backward).  Either way 16 products a thread in pairs, then one small sum.
+// Pairs because instructions count: the SMs issue every other cycle over the
+// whole solve (ncu, 48^3: 51 % of the slots).  20^3 57 -> 49 us, 33x35x37 94 ->
+// 82, 46^3 161 -> 148, 64^3 492 -> 467 against one row a thread and gathers in
+// fours.
+SPX_DEV int log2_at_least(int v) { return v <= 1 ? 0 : 32 - __clz(v - 1); }
+SPX_DEV int pow2_at_least(int v) { return 1 << log2_at_least(v); }
+// two adjacent rows of the tile (the swizzle keeps aligned groups of four)
+SPX_DEV double2 ld_pair(const double *p) { return *reinterpret_cast<const double2 *>(p); }
+SPX_DEV double2 ld_pair(const float *p) {
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    return make_double2(v.x, v.y);
+}
 
 SPX_DEV void vec_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &next, SNext<1> &nx,
                      uint32_t ph, SShared<1> &sh) {
@@ -346,18 +354,23 @@ SPX_DEV void vec_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
     nx.read(a);
     mbar_wait(&sh.pfull, ph, a.err);
     __syncthreads();
-    const int row = t & 15, grp = t >> 4, nb2 = pow2_at_least(k.nrb), P = kVecThreads / 16 / nb2;
-    const int rb = grp & (nb2 - 1), p = grp / nb2;
-    double acc = 0.0;
+    const int row = 2 * (t & 7), grp = t >> 3, lb = log2_at_least(k.nrb), P = kVecThreads / 8 >> lb;
+    const int rb = grp & ((1 << lb) - 1), p = grp >> lb;
+    double2 acc = make_double2(0.0, 0.0);
     if (rb < k.nrb) {
         const Real *G = sh.panel + rb * jn * 16;
-        for (int j = p; j < jn; j += P) acc += (double)G[j * 16 + (row ^ gswz(j0 + j))] * sh.vec[j];
+        for (int j = p; j < jn; j += P) {
+            const double2 g = ld_pair(G + j * 16 + (row ^ gswz(j0 + j)));
+            const double v = sh.vec[j];
+            acc.x += g.x * v;
+            acc.y += g.y * v;
+        }
     }
-    sh.part[p * nb2 * 16 + rb * 16 + row] = acc;
+    *reinterpret_cast<double2 *>(sh.part + (p << lb) * 16 + rb * 16 + row) = acc;
     __syncthreads();
     if (t < k.nrow) {
         double own = 0.0;
-        for (int q = 0; q < P; q++) own += sh.part[q * nb2 * 16 + t];
+        for (int q = 0; q < P; q++) own += sh.part[(q << lb) * 16 + t];
         if (k.strip < k.nstrip - 1) {
             put(w, a.o_fp + (int64_t)(k.slot0 + k.strip) * kVecRows + t, own);
         } else {
@@ -388,8 +401,11 @@ SPX_DEV void vec_bwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
 #pragma unroll
     for (int q = 0; q < Q; q++) {
         const int i = t + q * kVecThreads, ii = k.i0 + i;
-        src[q] = w.cur + (ii < k.c ? a.o_yf + k.first + ii : a.o_x + (i < k.nrow ? l.rows[i] : 0));
-        v[q] = i < k.nrow ? ld_val(src[q]) : 0.0;
+        v[q] = 0.0;
+        if (i < k.nrow) {
+            src[q] = w.cur + (ii < k.c ? a.o_yf + k.first + ii : a.o_x + l.rows[i]);
+            v[q] = ld_val(src[q]);
+        }
     }
 #pragma unroll
     for (int q = 0; q < Q; q++) {
@@ -403,15 +419,21 @@ SPX_DEV void vec_bwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
     nx.read(a);
     mbar_wait(&sh.pfull, ph, a.err);
     __syncthreads();
-    const int row = t & 15, grp = t >> 4, w2 = min(kVecThreads / 16, pow2_at_least(jn)), P = kVecThreads / 16 / w2;
-    const int p = grp / w2;
+    const int row = 2 * (t & 7), grp = t >> 3, lw = min(4, log2_at_least(jn));
+    const int w2 = 1 << lw, P = kVecThreads / 8 >> lw, p = grp >> lw;
+    static_assert(kVecThreads == 128, "16 groups");
     for (int j = grp & (w2 - 1); j < jn; j += w2) {
         double acc = 0.0;
-        const int rr = row ^ gswz(k.j0 + j);
-        for (int b = p; b < k.nrb; b += P) acc += (double)sh.panel[(b * jn + j) * 16 + rr] * sh.vec[b * 16 + row];
-        const unsigned half = 0xffffu << (t & 16);
+        const Real *G = sh.panel + j * 16 + (row ^ gswz(k.j0 + j));
+        for (int b = p; b < k.nrb; b += P) {
+            const double2 g = ld_pair(G + b * jn * 16);
+            const double2 v = *reinterpret_cast<const double2 *>(sh.vec + b * 16 + row);
+            acc += g.x * v.x;
+            acc += g.y * v.y;
+        }
+        const unsigned part = 0xffu << (t & 24);
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(half, acc, o);
+        for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(part, acc, o);
         if (row == 0) sh.part[p * w2 + j] = acc;
     }
     __syncthreads();
