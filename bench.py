@@ -457,13 +457,13 @@ def run_metric(args, pkg, wl, ctx):
                      "d2h_bytes_per_step": int(d2h), "steps_s": [round(x, 4) for x in ts]}
 
     # ---- roofline of the dominant kernel of the timed form.  For a block
-    # form that is the block solve mf_bsolve (FP32 panels in the mixed
+    # form that is the block solve mf_solve<NR> (FP32 panels in the mixed
     # form): algorithmic bytes of one launch (the plan's solve-pair bytes
     # with rows of b values) over its average device time, measured by the
     # library with CUDA events around every block solve of the timed solve
     # (t_block_solve over the solves that ran; corrections that returned at
     # once on the device add a few microseconds each).  For the
-    # single-vector forms it is the solve pair mf_solve_sf, timed the same
+    # single-vector forms it is the solve pair mf_solve<1>, timed the same
     # way through the operator phase.
     kt = keep[target]
     ei, info = kt["ei"], kt["info"]
@@ -472,12 +472,12 @@ def run_metric(args, pkg, wl, ctx):
         launches = max(1, int(ei["block_solves"]))
         per_launch = block_solve_bytes(kt["costs"]["op_bytes"], n, bsz)
         avg_s = float(ei["t_block_solve"]) / launches
-        kname = f"mf_bsolve<{(bsz + 7) // 8 * 8}>"
+        kname = f"mf_solve<{(bsz + 7) // 8 * 8}>"
     else:
         launches = max(1, int(info["nops"]) + int(ei["refine_steps"]))
         per_launch = kt["costs"]["op_bytes"]
         avg_s = kt["t_op"] / launches
-        kname = "mf_solve_sf"
+        kname = "mf_solve<1>"
     achieved = per_launch / avg_s / 1e9 if avg_s > 0 else None
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
@@ -1002,7 +1002,7 @@ def main():
             "data": "synthetic",
             "config": {"workload": wl["desc"], "n": int(n), "nnz": int(A.nnz), "k": k, "tol": TOL,
                        "precision": "plain FP64" if args.precision == "fp64" else
-                       "mixed: FP32 factor (TF32 tensor-core updates) + FP64 refinement",
+                       "mixed: FP32 factor + FP64 refinement",
                        "parallelism": f"replicas x{world}",
                        "l2": "256 MiB buffer written between timed steps",
                        "value_scope": "numeric factor + Lanczos, matrix and analysis resident"},

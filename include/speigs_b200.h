@@ -19,9 +19,9 @@ extern "C" {
 
 /* ---- extension options: precision of the shift-invert operator ------------
  * SPEIGS_B200_FP64: the drop-in path, an FP64 supernodal factor.
- * SPEIGS_B200_MIXED ('sm' only): the factor is stored in FP32 and its
- * trailing updates run on the TF32 tensor cores with an FP32-accurate
- * three-term split; every solve is refined in FP64 (r = b - (A+dI)y,
+ * SPEIGS_B200_MIXED ('sm' only): the factor is stored in FP32 (its products
+ * are FP64 products of FP32 tiles); every solve is refined in FP64
+ * (r = b - (A+dI)y,
  * y += M^{-1} r) until ||r|| <= refine_tol * (||A||_1 ||y|| + ||b||) or
  * refine_max corrections were made.  The Lanczos recurrence, the
  * reorthogonalisation, the Ritz problem and the residuals stay FP64.

@@ -28,9 +28,8 @@ struct SolvePlan {      // one tile queue of the solve
 };
 
 // Real is the storage type of the fronts and of the panels G: double for
-// the plain FP64 operator, float for the mixed-precision one (FP32 factor,
-// trailing updates on the TF32 tensor cores with an FP32-accurate 3-term
-// split; the caller refines each solve in FP64).  Vectors are FP64 always.
+// the plain FP64 operator, float for the mixed-precision one (FP64 products of
+// FP32 tiles; the caller refines each solve in FP64).  Vectors are FP64 always.
 template <class Real>
 class MultifrontalPlanT {
 public:
