@@ -133,6 +133,18 @@ struct TsParams {
     unsigned *counter;
 };
 
+// Shared memory beyond what a kernel may have unasked, 48 KB for its static
+// part (16 and 272 bytes in the kernels below) and the dynamic one together.
+// What may be asked for belongs to the kernel and the process, so every call
+// raises it to the same size, all that a block can have: with sizes of their
+// own, one thread's call could lower another's before its launch.
+constexpr size_t kSmemUnasked = 47 * 1024, kSmemMost = 227 * 1024 - 512;
+template <class... P>
+static void allow_smem(void (*kernel)(P...), size_t smem) {
+    if (smem > kSmemUnasked)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost);
+}
+
 // Final cross-block reduction by the last block to arrive: column c of the
 // partials (nb values in a row for each column) is summed by one warp in a
 // fixed order, so results are reproducible run to run.  A chain of one L2
@@ -596,10 +608,9 @@ void launch_ritz_vectors(const double *V, int64_t ldv, int n, int m, const doubl
                      nrm2 + v0, rs.part, rs.counter};
         const int nb = std::min(ts_blocks(n), kTsMaxBlocks);
         const size_t smem = sizeof(double) * (size_t)(m + kTsThreads / 32) * nvp;
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(vec ? ritz_kernel<true> : ritz_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        launch_chained(vec ? ritz_kernel<true> : ritz_kernel<false>, nb, kTsThreads, smem, st, p);
+        const auto kernel = vec ? ritz_kernel<true> : ritz_kernel<false>;
+        allow_smem(kernel, smem);
+        launch_chained(kernel, nb, kTsThreads, smem, st, p);
     }
 }
 
