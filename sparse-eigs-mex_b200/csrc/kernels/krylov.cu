@@ -453,11 +453,9 @@ static void ts_launch(const TsParams &p, cudaStream_t st) {
     const int slots = MODE == TS_DOT || MODE == TS_UPDATE_DOT ? p.m * ts_shares(p.m, per) : 0;
     const size_t smem = sizeof(double) * ((size_t)kGsSeg + ((p.m + 1) & ~1) + slots);
     const bool vec = (((uintptr_t)p.V | (uintptr_t)p.w) & 15u) == 0 && p.ldv % 2 == 0;
-    if (smem > 48 * 1024)                               // more than 1000 columns
-        cudaFuncSetAttribute(vec ? ts_kernel<MODE, true> : ts_kernel<MODE, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_chained(vec ? ts_kernel<MODE, true> : ts_kernel<MODE, false>, nb, kGsThreads, smem, st,
-                   p, per);
+    const auto kernel = vec ? ts_kernel<MODE, true> : ts_kernel<MODE, false>;
+    allow_smem(kernel, smem);                           // from about 960 columns on
+    launch_chained(kernel, nb, kGsThreads, smem, st, p, per);
 }
 
 void launch_ts_dot(const double *V, int64_t ldv, int n, int m, const double *w, double *h,

@@ -1,6 +1,7 @@
-"""Ritz vectors at the basis sizes where the kernel's static and dynamic shared memory pass 48 KB
-together: 120, 184, 248, 376 and 760 columns (wanted pairs in the residual test, k + 5 in the
-restart, single vectors and blocks).
+"""Ritz vectors and Gram-Schmidt passes at the basis sizes where a kernel's static and dynamic
+shared memory pass 48 KB together: Ritz vectors of 120, 184, 248, 376 and 760 columns (wanted
+pairs in the residual test, k + 5 in the restart, single vectors and blocks), dot products of
+1,023 and 1,024 columns.
 
 The matrix is tridiagonal: a uniformly distributed diagonal and a weak chain, whose largest
 values take several restarts; its eigenvalues come from SciPy's tridiagonal solver.  The solver
@@ -50,3 +51,16 @@ def test_ritz_vectors_of_blocks(pkg, lib, ncv, k):
     assert rc == 0, s.last_error(lib)
     assert einfo["block"] == 8 and info["nconv"] == k and info["flag"] == 0
     _check(A, lam, V, w[:k])
+
+
+def test_gram_schmidt_of_a_thousand_columns(pkg, lib):
+    """Every pair of a matrix of order 1,026 from a basis as large as it: a pass left out at any
+    width leaves pairs unconverged."""
+    s = pkg.speigs
+    n = 1026
+    A, w = _matrix(n)
+    rc, lam, V, _, info = s.speigs(
+        A, n, s.LM, s.default_opts(lib, tol=1e-10, ncv=n, maxit=1, dense_max=0, detect=0), lib=lib)
+    assert rc == 0, s.last_error(lib)
+    assert info["nconv"] == n and info["flag"] == 0 and info["restarts"] == 0
+    _check(A, lam, V, w)
