@@ -17,9 +17,10 @@ SPX_DEV void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A launch on `st`, chained or plain; what the runtime says to it.
 template <class... P, class... A>
-void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st,
-                    A... args) {
+cudaError_t launch_as(bool chained, void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                      cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -29,9 +30,20 @@ void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, c
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    cfg.numAttrs = chained ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
     note_launch();
+    return e;
+}
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                           cudaStream_t st, A... args) {
+    return launch_as(true, kernel, grid, threads, smem, st, args...);
+}
+template <class... P, class... A>
+cudaError_t launch_plain(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                         cudaStream_t st, A... args) {
+    return launch_as(false, kernel, grid, threads, smem, st, args...);
 }
 
 }  // namespace spx

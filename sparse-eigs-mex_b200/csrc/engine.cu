@@ -2387,7 +2387,7 @@ __global__ void densify_kernel(int n, const int32_t *rp, const int32_t *ci, cons
 // A few eigenpairs by reduction to tridiagonal form (dense_eig.cuh).  Returns 0
 // with lambda (sorted by |lambda|) and V, a negative code, or 1 when the
 // Jacobi solver has to do it: an entry out of the range whose squares are
-// safe, or pairs that miss the check of their residuals.
+// safe, a refused launch, or pairs that miss the check of their residuals.
 static int dense_few_pairs(int n, const double *D, int k, speigs_which which, double amax,
                            double *lambda, double *V, Arena &ar, cudaStream_t st) {
     if (n < kDenseEigMin || n > kDenseEigMax || k > kDenseEigMaxK || !(amax < 1e100) ||
@@ -2400,11 +2400,14 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
     int *ti = ar.alloc<int>(2 * (size_t)k);
     double *Z = ar.alloc<double>((size_t)n * k);
     if (ar.failed) return SPEIGS_ERR_MEM;
-    if (launch_dense_tridiag(n, D, Q, tb, td, te, work, st) != cudaSuccess) {
-        cudaGetLastError();          // a cluster of that size is not to be had
+    // a launch that is refused (no cluster of that size to be had, say)
+    auto refused = [](cudaError_t e) {
+        if (e != cudaSuccess) cudaGetLastError();
+        return e != cudaSuccess;
+    };
+    if (refused(launch_dense_tridiag(n, D, Q, tb, td, te, work, st)) ||
+        refused(launch_tri_bisect(n, td, te, k, which == SPEIGS_SM, tv, ti, st)))
         return 1;
-    }
-    launch_tri_bisect(n, td, te, k, which == SPEIGS_SM, tv, ti, st);
     std::vector<double> h(2 * (size_t)n + 2 * (size_t)k);
     std::vector<int> hi(2 * (size_t)k);
     copy_async(h.data(), td, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, st);
@@ -2434,8 +2437,9 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
     for (int t = 0; t < k; t++) lam[t] = cand[pick[t]];
     if (tri_vectors_host(n, h.data(), h.data() + n, k, lam.data(), zh.data()) != 0) return 1;
     copy_async(Z, zh.data(), sizeof(double) * (size_t)n * k, cudaMemcpyHostToDevice, st);
-    launch_apply_reflectors(n, Q, tb, Z, k, st);
-    launch_rayleigh_dd(n, D, Z, k, tl, tr, st);
+    if (refused(launch_apply_reflectors(n, Q, tb, Z, k, st)) ||
+        refused(launch_rayleigh_dd(n, D, Z, k, tl, tr, st)))
+        return 1;
     std::vector<double> q(2 * (size_t)k);
     copy_async(q.data(), tl, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);

@@ -1,5 +1,6 @@
 // See dense_eig.cuh.
 #include "dense_eig.cuh"
+#include "../chain.cuh"
 #include "../common.cuh"
 #include "../counters.h"
 
@@ -44,8 +45,9 @@ bool dense_tridiag_work(int n) { return tri_smem(n, kTriCluster) > kTriMaxSmem; 
 // The barrier and the reductions' latency are what bounds it (3 us a step at
 // n = 210, the products are 0.1 us), so the matrix stays in shared memory.  n =
 // 210: 868 us with a second barrier a step (the owner made the reflector and
-// distributed it) and 8 blocks, 696 with one barrier, 645 with 16 blocks.  The Jacobi solver took 95 ms, all of it on one SM and, from n = 110,
-// out of global memory.
+// distributed it) and 8 blocks, 696 with one barrier, 645 with 16 blocks.  The
+// Jacobi solver took 95 ms, all of it on one SM and, from n = 110, out of
+// global memory.
 __global__ void __launch_bounds__(kTriThreads)
 dense_tridiag_kernel(int n, const double *__restrict__ D, double *__restrict__ V,
                      double *__restrict__ beta, double *__restrict__ d, double *__restrict__ e,
@@ -190,6 +192,17 @@ cudaError_t launch_dense_tridiag(int n, const double *D, double *V, double *beta
     return err;
 }
 
+// The kernels below hold one or two vectors in dynamic shared memory.  Up to
+// 48 KB, static and dynamic part together (20.7 KB of the quotients' is
+// static), need no asking; what is asked for is the largest order's size
+// whatever n is, since it belongs to the kernel and the process: with the size
+// of each call, one thread's call could lower another's before its launch.
+template <class... P>
+static cudaError_t allow_vectors(void (*kernel)(P...)) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(double) * 2 * kDenseEigMax));
+}
+
 // ------------------------------------------------------------ bisection --
 // eigenvalues of (d, e) below x (Sturm count of the LDL^T pivots)
 SPX_DEV int sturm(int n, const double *d, const double *e2, double pivmin, double x) {
@@ -275,13 +288,11 @@ tri_bisect_kernel(int n, const double *__restrict__ gd, const double *__restrict
     }
 }
 
-void launch_tri_bisect(int n, const double *d, const double *e, int k, bool smallest, double *val,
-                       int *idx, cudaStream_t st) {
-    const size_t smem = sizeof(double) * 2 * (size_t)n;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(tri_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    tri_bisect_kernel<<<2 * k, kBisThreads, smem, st>>>(n, d, e, k, smallest, val, idx);
-    note_launch();
+cudaError_t launch_tri_bisect(int n, const double *d, const double *e, int k, bool smallest,
+                              double *val, int *idx, cudaStream_t st) {
+    if (cudaError_t err = allow_vectors(tri_bisect_kernel)) return err;
+    return launch_plain(tri_bisect_kernel, 2 * k, kBisThreads, sizeof(double) * 2 * (size_t)n, st, n,
+                        d, e, k, smallest, val, idx);
 }
 
 // ------------------------------------------------------- back-transform --
@@ -326,13 +337,12 @@ apply_reflectors_kernel(int n, const double *__restrict__ V, const double *__res
         if (tid + 128 * q < n) z[tid + 128 * q] = x[q];
 }
 
-void launch_apply_reflectors(int n, const double *V, const double *beta, double *Z, int nc,
-                             cudaStream_t st) {
-    if (n < 3 || nc <= 0) return;
-    if (n <= 256) apply_reflectors_kernel<2><<<nc, 128, 0, st>>>(n, V, beta, Z);
-    else if (n <= 1024) apply_reflectors_kernel<8><<<nc, 128, 0, st>>>(n, V, beta, Z);
-    else apply_reflectors_kernel<32><<<nc, 128, 0, st>>>(n, V, beta, Z);
-    note_launch();
+cudaError_t launch_apply_reflectors(int n, const double *V, const double *beta, double *Z, int nc,
+                                    cudaStream_t st) {
+    if (n < 3 || nc <= 0) return cudaSuccess;
+    const auto kernel = n <= 256 ? apply_reflectors_kernel<2>
+                        : n <= 1024 ? apply_reflectors_kernel<8> : apply_reflectors_kernel<32>;
+    return launch_plain(kernel, nc, 128, 0, st, n, V, beta, Z);
 }
 
 // ----------------------------------------- quotients in twice the precision --
@@ -426,13 +436,11 @@ rayleigh_dd_kernel(int n, const double *__restrict__ D, const double *__restrict
     }
 }
 
-void launch_rayleigh_dd(int n, const double *D, const double *X, int nc, double *lam, double *res2,
-                        cudaStream_t st) {
-    const size_t smem = sizeof(double) * 2 * (size_t)n;
-    if (smem > 32 * 1024)
-        cudaFuncSetAttribute(rayleigh_dd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    rayleigh_dd_kernel<<<nc, kRayThreads, smem, st>>>(n, D, X, lam, res2);
-    note_launch();
+cudaError_t launch_rayleigh_dd(int n, const double *D, const double *X, int nc, double *lam,
+                               double *res2, cudaStream_t st) {
+    if (cudaError_t err = allow_vectors(rayleigh_dd_kernel)) return err;
+    return launch_plain(rayleigh_dd_kernel, nc, kRayThreads, sizeof(double) * 2 * (size_t)n, st, n, D,
+                        X, lam, res2);
 }
 
 }  // namespace spx

@@ -15,6 +15,9 @@ constexpr int kDenseEigMin = 24;     // smaller orders: the Jacobi solver
 constexpr int kDenseEigMax = 4096;   // the back-transformation's registers
 constexpr int kDenseEigMaxK = 64;    // more vectors: the Jacobi solver
 
+// The launchers return what the runtime says to the launch; after a refused
+// one nothing has been written.
+
 // D (n x n, full symmetric, kept) -> T = Q^T D Q: d[n], e[n-1], reflector k
 // (I - beta[k] v v^T) in column k of V below the diagonal (n x n, ld n).
 // work: n x n doubles, used when the matrix does not fit the cluster's shared
@@ -26,16 +29,16 @@ cudaError_t launch_dense_tridiag(int n, const double *D, double *V, double *beta
 // Eigenvalues of the tridiagonal (d, e): the 2k around zero (smallest) or the
 // k lowest and k highest (else), val[2k] with their ascending positions in
 // idx[2k]; -1 where there is none (2k > n).
-void launch_tri_bisect(int n, const double *d, const double *e, int k, bool smallest, double *val,
-                       int *idx, cudaStream_t st);
+cudaError_t launch_tri_bisect(int n, const double *d, const double *e, int k, bool smallest,
+                              double *val, int *idx, cudaStream_t st);
 
 // Z (n x nc, ld n) := Q Z
-void launch_apply_reflectors(int n, const double *V, const double *beta, double *Z, int nc,
-                             cudaStream_t st);
+cudaError_t launch_apply_reflectors(int n, const double *V, const double *beta, double *Z, int nc,
+                                    cudaStream_t st);
 
 // Rayleigh quotients of the columns of X, accumulated in twice the working
 // precision, and the squared residual norms ||D x - lambda x||^2 / ||x||^2
-void launch_rayleigh_dd(int n, const double *D, const double *X, int nc, double *lam, double *res2,
-                        cudaStream_t st);
+cudaError_t launch_rayleigh_dd(int n, const double *D, const double *X, int nc, double *lam,
+                               double *res2, cudaStream_t st);
 
 }  // namespace spx
