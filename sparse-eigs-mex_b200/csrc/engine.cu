@@ -45,6 +45,11 @@ static cudaError_t copy_async(void *dst, const void *src, size_t bytes, cudaMemc
 
 static thread_local char g_err[256] = "";
 const char *last_cuda_error() { return g_err; }
+// what an earlier call of this thread left behind
+static void begin_call() {
+    g_err[0] = 0;
+    launch_error() = cudaSuccess;
+}
 const char *set_last_error_text(const char *msg) {
     snprintf(g_err, sizeof g_err, "%s", msg);
     return g_err;
@@ -106,7 +111,7 @@ static int syev_projected(int m, const double *dH, int ldh, double *dtheta, doub
     note_d2h((long long)sizeof(double) * m * m);
     cudaMemcpy2DAsync(hH, sizeof(double) * m, dH, sizeof(double) * ldh, sizeof(double) * m, m,
                       cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "projected problem read-back");
     // nvec >= 0: eigenvectors only for the nvec wanted Ritz values (the
     // rest of S is zero); the eigenvalues are those of the full solver
@@ -564,7 +569,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
     auto read_nrm = [&](double *out) -> int {
         copy_async(h_nrm, b.nrm2, sizeof(double), cudaMemcpyDeviceToHost, st);
         if (op_err) copy_async(h_operr, op_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "lanczos sync");
         tm.resolve();
         if (op_err && *h_operr) {
@@ -663,7 +668,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
         cudaEventRecord(evb.e[jj & 1], st);
     };
     auto wait_beta = [&](int64_t jj, double *beta) -> int {
-        cudaError_t e = cudaEventSynchronize(evb.e[jj & 1]);
+        cudaError_t e = launch_result(cudaEventSynchronize(evb.e[jj & 1]));
         if (e != cudaSuccess) return cuda_fail(e, "lanczos sync");
         if (op_err && h_sterr[jj & 1]) {
             set_last_error_text("operator application failed: a solve dependency wait ran out");
@@ -673,7 +678,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
         return 0;
     };
     auto drain = [&]() -> int {
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "lanczos sync");
         tm.resolve();
         return 0;
@@ -734,7 +739,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
         copy_async(h_r2, b.r2, sizeof(double) * nwant, cudaMemcpyDeviceToHost, st);
         copy_async(jst, b.jstat, sizeof(int), cudaMemcpyDeviceToHost, st);
         {
-            cudaError_t e = cudaStreamSynchronize(st);
+            cudaError_t e = launch_result(cudaStreamSynchronize(st));
             if (e != cudaSuccess) return cuda_fail(e, "residual sync");
             tm.resolve();
         }
@@ -821,7 +826,7 @@ static int lanczos_device(Operator &op, const DevA &A, int n, int64_t k, const s
     *ldx = b.ldv;
     *nout = last_nwant;
     {
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "lanczos end");
         tm.resolve();
     }
@@ -952,7 +957,7 @@ static int block_lanczos_device(BlockOperator &op, const DevA &A, int n, int64_t
     op.ms_solve = &op.ms_solve_acc;
     auto sync = [&](const char *where) -> int {
         if (op_err) copy_async(h_operr, op_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, where);
         tm.resolve();
         if (op_err && *h_operr) {
@@ -1411,7 +1416,7 @@ static int plan_upload_values(speigs_plan_s *p) {
     cudaError_t e = copy_async(p->d_va, p->A.val, sizeof(double) * nnz,
                                     cudaMemcpyHostToDevice, p->stream.s);
     if (e != cudaSuccess) return cuda_fail(e, "upload values");
-    e = cudaStreamSynchronize(p->stream.s);
+    e = launch_result(cudaStreamSynchronize(p->stream.s));
     if (e != cudaSuccess) return cuda_fail(e, "upload values");
     p->factored = false;
     return 0;
@@ -1431,7 +1436,7 @@ static int plan_alloc(speigs_plan_s *p, void **ptr, size_t bytes) {
 // Build the plan from an already expanded full CSR (takes ownership of A).
 int plan_from_csr(HostCSR &A, speigs_which which, const speigs_opts &o, double anorm,
                   const speigs_ext_opts *ext, speigs_plan_s **out) {
-    g_err[0] = 0;
+    begin_call();
     int ndev = 0;
     cudaError_t e0 = cudaGetDeviceCount(&ndev);
     if (e0 != cudaSuccess || ndev == 0) {
@@ -1518,7 +1523,7 @@ static int plan_dense_inverse(speigs_plan_s *p) {
     if (ar.failed) return SPEIGS_ERR_MEM;
     launch_dense_inverse(n, p->d_rp, p->d_ci, p->d_va, p->anorm, p->d_ainv, rowbuf, colbuf, ipiv,
                          flags, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "dense inverse");
     return 0;
 }
@@ -1601,7 +1606,7 @@ static double *pinned_scalars(size_t need) {
 // device buffers.
 static int plan_solve(speigs_plan_s *p, int64_t k, double *lambda, double *V, double *resid,
                       speigs_info *info, bool on_device, EngineStats *stats) {
-    g_err[0] = 0;
+    begin_call();
     cudaStream_t st = p->stream.s;
     const int n = p->A.n;
     if (k <= 0 || k > n) return SPEIGS_ERR_ARG;
@@ -1664,7 +1669,8 @@ static int plan_solve(speigs_plan_s *p, int64_t k, double *lambda, double *V, do
                 kind = cudaMemcpyDeviceToDevice;
             cudaGetLastError();
             copy_async(dw, p->ext_warm, sizeof(double) * (size_t)n * wcols, kind, st);
-            if (cudaError_t e = cudaStreamSynchronize(st)) return cuda_fail(e, "start subspace upload");
+            if (cudaError_t e = launch_result(cudaStreamSynchronize(st)))
+                return cuda_fail(e, "start subspace upload");
             dwarm = dw;
         }
         const double ti = wall();
@@ -1762,7 +1768,7 @@ static int plan_solve(speigs_plan_s *p, int64_t k, double *lambda, double *V, do
                 memcpy(lambda, ls.data(), sizeof(double) * nout);
                 if (resid) memcpy(resid, rs.data(), sizeof(double) * nout);
             }
-            cudaError_t e = cudaStreamSynchronize(st);
+            cudaError_t e = launch_result(cudaStreamSynchronize(st));
             if (e != cudaSuccess) rc = cuda_fail(e, "copy out");
         }
         info->t_iter = wall() - ti;
@@ -1982,7 +1988,7 @@ int device_batched_krylov(HostCSR &A, int nseg, const int32_t *off_h, int64_t k,
                           double *lam_out, double *res_out, double *X_out, int64_t *nconv_out,
                           int64_t *nops_out, int64_t *restarts_out, int *flag_out,
                           BatchedStats *bst, int *handed, int handoff) {
-    g_err[0] = 0;
+    begin_call();
     const int n = A.n;
     if (handed) std::fill(handed, handed + nseg, 0);
     double amax = 1.0;
@@ -2074,7 +2080,7 @@ int device_batched_krylov(HostCSR &A, int nseg, const int32_t *off_h, int64_t k,
         cudaMemsetAsync(a.err, 0, sizeof(int), st);
         cudaMemsetAsync(a.X, 0, sizeof(double) * (size_t)a.ldv * k, st);
         cudaMemsetAsync(a.x, 0, sizeof(double) * (size_t)a.ldv, st);
-        cudaError_t e = cudaStreamSynchronize(st);   // the host vectors die here
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));   // the host vectors die here
         if (e != cudaSuccess) return cuda_fail(e, "batched set-up");
     }
     const uint64_t seed = o.seed ? o.seed : 88172645463325252ULL;
@@ -2117,7 +2123,7 @@ int device_batched_krylov(HostCSR &A, int nseg, const int32_t *off_h, int64_t k,
     auto sync_read = [&](const char *where) -> int {
         copy_async(&herr[0], a.err, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (op_err) copy_async(&herr[1], op_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, where);
         if (herr[0]) { set_last_error_text("a start vector has zero norm"); return SPEIGS_ERR_INTERNAL; }
         if (herr[1]) {
@@ -2242,7 +2248,7 @@ __global__ void times_i_kernel(int n, const double *w, double *dst) {
 int device_hermitian_recover(int64_t n64, int64_t kk, int64_t k, const double *V2,
                              const double *lam2, const double *res2, double *lambda, double *Vr,
                              double *Vi, double *resid, int64_t *nacc_out) {
-    g_err[0] = 0;
+    begin_call();
     if (2 * n64 > INT32_MAX) return SPEIGS_ERR_ARG;
     const int n = (int)n64, n2 = 2 * n;
     Stream stream;
@@ -2270,7 +2276,7 @@ int device_hermitian_recover(int64_t n64, int64_t kk, int64_t k, const double *V
         copy_async(C, V2, sizeof(double) * (size_t)n2 * kk, cudaMemcpyHostToDevice, st);
         auto read_nrm = [&](double *out) -> int {
             copy_async(hn, nrm2, sizeof(double), cudaMemcpyDeviceToHost, st);
-            cudaError_t e = cudaStreamSynchronize(st);
+            cudaError_t e = launch_result(cudaStreamSynchronize(st));
             if (e != cudaSuccess) return cuda_fail(e, "hermitian recovery");
             *out = std::sqrt(hn[0]);
             return 0;
@@ -2310,7 +2316,7 @@ int device_hermitian_recover(int64_t n64, int64_t kk, int64_t k, const double *V
             if (Vi) copy_async(Vi + (size_t)a * n, u + n, sizeof(double) * n,
                                cudaMemcpyDeviceToHost, st);
         }
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "hermitian recovery");
     }
     for (int64_t a = 0; a < nacc; a++) {
@@ -2333,7 +2339,7 @@ __global__ void absbits_kernel(int n, const double *d, unsigned long long *key, 
 
 int device_diag_path(int64_t n64, const double *diag, int64_t k, speigs_which which,
                      double *lambda, double *V, double *resid, speigs_info *info) {
-    g_err[0] = 0;
+    begin_call();
     if (n64 > INT32_MAX) return SPEIGS_ERR_ARG;
     const int n = (int)n64;
     Stream stream;
@@ -2361,7 +2367,7 @@ int device_diag_path(int64_t n64, const double *diag, int64_t k, speigs_which wh
         else
             cub::DeviceRadixSort::SortPairsDescending(tmp, tb, k0, k1, i0, i1, n, 0, 64, st);
         copy_async(ord.data(), i1, sizeof(int) * k, cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "diag sort");
     }
     for (int64_t t = 0; t < k; t++) {
@@ -2402,8 +2408,9 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
     if (ar.failed) return SPEIGS_ERR_MEM;
     // a launch that is refused (no cluster of that size to be had, say)
     auto refused = [](cudaError_t e) {
-        if (e != cudaSuccess) cudaGetLastError();
-        return e != cudaSuccess;
+        if (e == cudaSuccess) return false;
+        launch_result(cudaGetLastError());
+        return true;
     };
     if (refused(launch_dense_tridiag(n, D, Q, tb, td, te, work, st)) ||
         refused(launch_tri_bisect(n, td, te, k, which == SPEIGS_SM, tv, ti, st)))
@@ -2413,7 +2420,7 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
     copy_async(h.data(), td, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, st);
     copy_async(h.data() + 2 * n, tv, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, st);
     copy_async(hi.data(), ti, sizeof(int) * 2 * k, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "dense path");
     // the k wanted of the candidates (ascending, each once), by |theta|, ties
     // in ascending order
@@ -2442,7 +2449,7 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
         return 1;
     std::vector<double> q(2 * (size_t)k);
     copy_async(q.data(), tl, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost, st);
-    e = cudaStreamSynchronize(st);
+    e = launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "dense path");
     for (int t = 0; t < k; t++)
         if (!(sqrt(q[k + t]) <= 1e-13 * n * amax)) return 1;
@@ -2453,13 +2460,13 @@ static int dense_few_pairs(int n, const double *D, int k, speigs_which which, do
         if (V) copy_async(V + (size_t)t * n, Z + (size_t)o[t] * n, sizeof(double) * n,
                           cudaMemcpyDeviceToHost, st);
     }
-    e = cudaStreamSynchronize(st);
+    e = launch_result(cudaStreamSynchronize(st));
     return e == cudaSuccess ? 0 : cuda_fail(e, "dense path copy");
 }
 
 int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *lambda,
                       double *V, double *resid, speigs_info *info) {
-    g_err[0] = 0;
+    begin_call();
     const int n = A.n;
     const int64_t nnz = A.nnz();
     Stream stream;
@@ -2507,7 +2514,7 @@ int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *l
         int hst[2] = {0, 0};
         copy_async(theta.data(), th, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
         copy_async(hst, stt, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "dense path");
         if (hst[0] < 0) return SPEIGS_ERR_LAPACK;
         // order by |theta| ascending ('sm') or descending ('lm'), stable
@@ -2520,7 +2527,7 @@ int device_dense_path(const HostCSR &A, int64_t k, speigs_which which, double *l
             for (int64_t t = 0; t < k; t++)
                 copy_async(V + (size_t)t * n, S + (size_t)ordd[t] * n, sizeof(double) * n,
                                 cudaMemcpyDeviceToHost, st);
-        e = cudaStreamSynchronize(st);
+        e = launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "dense path copy");
     }
     for (int64_t t = 0; t < k; t++) {
@@ -2607,7 +2614,7 @@ static int plan_set_values_device(speigs_plan p, const double *Ax) {
         launch_csc_map(n, dAp, dAi, p->d_rp, p->d_ci, p->d_map, bad, st);
         int h_bad = 0;
         copy_async(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = cudaStreamSynchronize(st);
+        cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
         if (e != cudaSuccess) return cuda_fail(e, "value map");
         p->map_state = h_bad ? -1 : 1;
         if (h_bad) return 1;
@@ -2620,7 +2627,7 @@ static int plan_set_values_device(speigs_plan p, const double *Ax) {
     launch_csc_values(n, p->d_rp, p->d_map, p->d_ax, p->d_va, bits, st);
     double anorm = 0.0;
     copy_async(&anorm, bits, sizeof anorm, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "new values");
     p->anorm = anorm > 0 ? anorm : 1.0;
     return 0;
@@ -2628,6 +2635,7 @@ static int plan_set_values_device(speigs_plan p, const double *Ax) {
 
 int speigs_plan_set_values(speigs_plan p, const double *Ax) {
     if (!p || !Ax) return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     const int dev_rc = plan_set_values_device(p, Ax);
     if (dev_rc <= 0) return dev_rc;
     const int64_t n = p->A.n;
@@ -2653,6 +2661,7 @@ int speigs_plan_solve_device(speigs_plan p, speigs_int k, double *lambda, double
 int speigs_plan_factor(speigs_plan p, double *shift) {
     if (!p) return SPEIGS_ERR_ARG;
     if (p->which != SPEIGS_SM) return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     int rc = spx::plan_factor(p, nullptr);
     if (shift) *shift = p->shift;
     return rc;
@@ -2660,6 +2669,7 @@ int speigs_plan_factor(speigs_plan p, double *shift) {
 
 int speigs_plan_apply_device(speigs_plan p, const double *x, double *y) {
     if (!p || !x || !y) return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     cudaStream_t st = p->stream.s;
     if (p->which == SPEIGS_LM) {
         spx::launch_spmv(p->A.n, p->d_rp, p->d_ci, p->d_va, x, y, st);
@@ -2681,7 +2691,7 @@ int speigs_plan_apply_device(speigs_plan p, const double *x, double *y) {
     int herr = 0;
     if (p->which == SPEIGS_SM && !p->lu && p->mf.error_word())
         cudaMemcpyAsync(&herr, p->mf.error_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return spx::cuda_fail(e, "apply");
     if (herr) {
         spx::set_last_error_text("solve failed: a dependency wait ran out");
@@ -2694,6 +2704,7 @@ int speigs_plan_apply_block_device(speigs_plan p, const double *x, int64_t ldx, 
                                    int64_t ldy, int nr) {
     if (!p || !x || !y || nr < 1 || nr > spx::kBlockMaxB || ldx < p->A.n || ldy < p->A.n)
         return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     cudaStream_t st = p->stream.s;
     const int n = p->A.n;
     int rc = 0;
@@ -2726,7 +2737,8 @@ int speigs_plan_apply_block_device(speigs_plan p, const double *x, int64_t ldx, 
             spx::DevA dA{n, p->d_rp, p->d_ci, p->d_va};
             spx::BlockMixedOperator op(&p->mf, dA, p->shift, p->anorm, &brf);
             rc = op.apply(x, ldx, y, ldy, nr, st);
-            cudaError_t e = cudaStreamSynchronize(st);   // before the arena returns its memory
+            // before the arena returns its memory
+            cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
             if (!rc && e != cudaSuccess) rc = spx::cuda_fail(e, "apply block");
         } else {
             rc = p->mf.solve_block(x, ldx, y, ldy, nr, st);
@@ -2736,7 +2748,7 @@ int speigs_plan_apply_block_device(speigs_plan p, const double *x, int64_t ldx, 
     int herr = 0;
     if (p->which == SPEIGS_SM && !p->lu && p->mf.error_word())
         cudaMemcpyAsync(&herr, p->mf.error_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return spx::cuda_fail(e, "apply block");
     if (herr) {
         spx::set_last_error_text("solve failed: a dependency wait ran out");
@@ -2775,6 +2787,7 @@ void speigs_plan_destroy(speigs_plan p) {
 
 int speigs_b200_rand_vec(speigs_int n, uint64_t seed, double *v) {
     if (n <= 0 || n > INT32_MAX || !v) return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     spx::Stream s;
     if (s.err != cudaSuccess) return spx::cuda_fail(s.err, "stream");
     double *d = nullptr;
@@ -2785,12 +2798,13 @@ int speigs_b200_rand_vec(speigs_int n, uint64_t seed, double *v) {
     spx::launch_rand_vec((int)n, seed, d, s.s);
     spx::copy_async(v, d, sizeof(double) * n, cudaMemcpyDeviceToHost, s.s);
     cudaFreeAsync(d, s.s);
-    cudaError_t e = cudaStreamSynchronize(s.s);
+    cudaError_t e = spx::launch_result(cudaStreamSynchronize(s.s));
     return e == cudaSuccess ? SPEIGS_OK : spx::cuda_fail(e, "rand_vec");
 }
 
 int speigs_b200_syev_small(int m, const double *H, double *theta, double *S, int *ord) {
     if (m <= 0 || !H || !theta || !S || !ord) return SPEIGS_ERR_ARG;
+    spx::launch_error() = cudaSuccess;
     spx::Stream s;
     if (s.err != cudaSuccess) return spx::cuda_fail(s.err, "stream");
     const size_t mm = (size_t)m * m, me = (size_t)((m + 1) & ~1);
@@ -2814,7 +2828,7 @@ int speigs_b200_syev_small(int m, const double *H, double *theta, double *S, int
     }
     void *ptrs[] = {dH, dth, dS, dw, dord, dst};
     for (void *q : ptrs) if (q) cudaFreeAsync(q, s.s);
-    cudaError_t e = cudaStreamSynchronize(s.s);
+    cudaError_t e = spx::launch_result(cudaStreamSynchronize(s.s));
     if (e != cudaSuccess) return spx::cuda_fail(e, "syev_small");
     if (!rc && hst[0] < 0) rc = SPEIGS_ERR_LAPACK;
     return rc;

@@ -671,9 +671,11 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         rc = rc ? rc : dupload(&db, bent.data(), bent.size(), st);
         if (!rc) {
             const int nblk = (2 * ns + 3) / 4;
-            expand_tasks_kernel<<<nblk, 128, 0, st>>>(dn, dv, ns, true, d_cptr_, (STask *)d_vtask_);
-            expand_tasks_kernel<<<nblk, 128, 0, st>>>(dn, db, ns, false, d_cptr_, (STask *)d_btask_);
-            note_launch(2);
+            if (launch_plain(expand_tasks_kernel, nblk, 128, 0, st, dn, dv, ns, true, d_cptr_,
+                             (STask *)d_vtask_) != cudaSuccess ||
+                launch_plain(expand_tasks_kernel, nblk, 128, 0, st, dn, db, ns, false, d_cptr_,
+                             (STask *)d_btask_) != cudaSuccess)
+                rc = SPEIGS_ERR_INTERNAL;
         }
         if (dn) cudaFreeAsync(dn, st);
         if (dv) cudaFreeAsync(dv, st);
@@ -734,12 +736,12 @@ template <> int MultifrontalPlanT<Real>::factorize(const double *d_val, double s
     a.queue = a.upd + ns_;
     a.status = a.queue + 1;
     a.err = a.queue + 2;
-    mf_factor<<<std::min(factor_grid_, nftask_), kFThreads, sizeof(FShared), st>>>(a);
-    note_launch();
+    cudaError_t e = launch_plain(mf_factor, std::min(factor_grid_, nftask_), kFThreads,
+                                 sizeof(FShared), st, a);
     int h[2] = {0, 0};
     cudaMemcpyAsync(h, a.status, sizeof h, cudaMemcpyDeviceToHost, st);
     note_d2h(sizeof h);
-    cudaError_t e = cudaStreamSynchronize(st);
+    if (cudaError_t es = cudaStreamSynchronize(st)) e = es;
     if (e != cudaSuccess || h[1]) {
         cudaGetLastError();
         return SPEIGS_ERR_INTERNAL;
@@ -764,9 +766,8 @@ template <> int MultifrontalPlanT<Real>::solve_setup(int q, cudaStream_t st) {
                          (int64_t)p.bslots * kBwdCols) * nr;
     sstride_[q] = (len + 1) & ~(int64_t)1;
     if ((rc = dmalloc(&d_sval_[q], (size_t)sstride_[q] * 2, st))) return rc;
-    fill_unset_kernel<<<2 * 148, 256, 0, st>>>(d_sval_[q], 2 * sstride_[q]);
-    note_launch();
-    return 0;
+    return launch_plain(fill_unset_kernel, 2 * 148, 256, 0, st, d_sval_[q], 2 * sstride_[q]) ==
+                   cudaSuccess ? 0 : SPEIGS_ERR_INTERNAL;
 }
 
 template <> int MultifrontalPlanT<Real>::run_solve(int q, const double *B, int64_t ldb, double *X,
@@ -799,12 +800,13 @@ template <> int MultifrontalPlanT<Real>::run_solve(int q, const double *B, int64
     a.accumulate = accumulate ? 1 : 0;
     a.skip = skip;
     const int grid = std::min(sgrid_[q], a.ntasks);
-    if (q == 0) launch_chained(mf_solve<1>, grid, kVecThreads, sizeof(SShared<1>), st, a);
-    else if (q == 1) launch_chained(mf_solve<8>, grid, kBlkThreads, sizeof(SShared<8>), st, a);
-    else if (q == 2) launch_chained(mf_solve<16>, grid, kBlkThreads, sizeof(SShared<16>), st, a);
-    else if (q == 3) launch_chained(mf_solve<24>, grid, kBlkThreads, sizeof(SShared<24>), st, a);
-    else launch_chained(mf_solve<32>, grid, kBlkThreads, sizeof(SShared<32>), st, a);
-    return 0;
+    const cudaError_t e =
+        q == 0   ? launch_chained(mf_solve<1>, grid, kVecThreads, sizeof(SShared<1>), st, a)
+        : q == 1 ? launch_chained(mf_solve<8>, grid, kBlkThreads, sizeof(SShared<8>), st, a)
+        : q == 2 ? launch_chained(mf_solve<16>, grid, kBlkThreads, sizeof(SShared<16>), st, a)
+        : q == 3 ? launch_chained(mf_solve<24>, grid, kBlkThreads, sizeof(SShared<24>), st, a)
+                 : launch_chained(mf_solve<32>, grid, kBlkThreads, sizeof(SShared<32>), st, a);
+    return e == cudaSuccess ? 0 : SPEIGS_ERR_INTERNAL;
 }
 
 template <> void MultifrontalPlanT<Real>::solve(const double *b, double *x, cudaStream_t st,
