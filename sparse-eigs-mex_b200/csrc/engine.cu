@@ -2592,42 +2592,58 @@ int speigs_plan_create_ex(speigs_int n, const speigs_int *Ap, const speigs_int *
     return SPEIGS_OK;
 }
 
-// The device path of speigs_plan_set_values.  Returns 0, a negative code, or 1
-// when the host has to rebuild the CSR.
-static int plan_set_values_device(speigs_plan p, const double *Ax) {
+// The value map of plan_set_values_device, made at a plan's first new values.
+// Returns 0, a negative code, or 1 when there is none to be had: columns that
+// are not strictly sorted (for good), or no device memory for it (then the next
+// call tries again).  Without a map nothing stays allocated for it.
+static int plan_value_map(speigs_plan p) {
     using namespace spx;
     cudaStream_t st = p->stream.s;
     const int n = p->A.n;
     const int64_t nnz = p->A.nnz(), cnnz = (int64_t)p->Ai_copy.size();
     if (p->map_state < 0 || cnnz > INT32_MAX) return 1;
-    Arena ar(st);
-    if (p->map_state == 0) {
-        int rc = plan_alloc(p, (void **)&p->d_map, sizeof(int32_t) * nnz);
-        rc = rc ? rc : plan_alloc(p, (void **)&p->d_ax, sizeof(double) * cnnz);
-        if (rc) return rc;
+    if (p->map_state > 0) return 0;
+    const size_t owned = p->owned.size();
+    int h_bad = 1;
+    cudaError_t e = cudaSuccess;
+    {
+        Arena ar(st);
         int64_t *dAp = ar.alloc<int64_t>(n + 1), *dAi = ar.alloc<int64_t>(cnnz);
         int *bad = ar.alloc<int>(1);
-        if (ar.failed) return SPEIGS_ERR_MEM;
-        copy_async(dAp, p->Ap_copy.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
-        copy_async(dAi, p->Ai_copy.data(), sizeof(int64_t) * cnnz, cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(bad, 0, sizeof(int), st);
-        launch_csc_map(n, dAp, dAi, p->d_rp, p->d_ci, p->d_map, bad, st);
-        int h_bad = 0;
-        copy_async(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-        cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
-        if (e != cudaSuccess) return cuda_fail(e, "value map");
-        p->map_state = h_bad ? -1 : 1;
-        if (h_bad) return 1;
+        if (!ar.failed && plan_alloc(p, (void **)&p->d_map, sizeof(int32_t) * nnz) == 0 &&
+            plan_alloc(p, (void **)&p->d_ax, sizeof(double) * cnnz) == 0) {
+            copy_async(dAp, p->Ap_copy.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
+            copy_async(dAi, p->Ai_copy.data(), sizeof(int64_t) * cnnz, cudaMemcpyHostToDevice, st);
+            cudaMemsetAsync(bad, 0, sizeof(int), st);
+            launch_csc_map(n, dAp, dAi, p->d_rp, p->d_ci, p->d_map, bad, st);
+            copy_async(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
+            e = launch_result(cudaStreamSynchronize(st));
+            p->map_state = e != cudaSuccess ? 0 : h_bad ? -1 : 1;
+        }
     }
+    if (p->map_state > 0) return 0;
+    for (; p->owned.size() > owned; p->owned.pop_back()) cudaFreeAsync(p->owned.back(), st);
+    p->d_map = nullptr;
+    p->d_ax = nullptr;
+    return e != cudaSuccess ? cuda_fail(e, "value map") : 1;
+}
+
+// The device path of speigs_plan_set_values.  Returns 0, a negative code, or 1
+// when the host has to rebuild the CSR.
+static int plan_set_values_device(speigs_plan p, const double *Ax) {
+    using namespace spx;
+    cudaStream_t st = p->stream.s;
+    if (int rc = plan_value_map(p)) return rc;
+    Arena ar(st);
     unsigned long long *bits = ar.alloc<unsigned long long>(1);
-    if (ar.failed) return SPEIGS_ERR_MEM;
+    if (ar.failed) return 1;
     p->factored = false;
     cudaMemsetAsync(bits, 0, sizeof *bits, st);
-    copy_async(p->d_ax, Ax, sizeof(double) * cnnz, cudaMemcpyHostToDevice, st);
-    launch_csc_values(n, p->d_rp, p->d_map, p->d_ax, p->d_va, bits, st);
+    copy_async(p->d_ax, Ax, sizeof(double) * p->Ai_copy.size(), cudaMemcpyHostToDevice, st);
+    launch_csc_values(p->A.n, p->d_rp, p->d_map, p->d_ax, p->d_va, bits, st);
     double anorm = 0.0;
     copy_async(&anorm, bits, sizeof anorm, cudaMemcpyDeviceToHost, st);
-    cudaError_t e = spx::launch_result(cudaStreamSynchronize(st));
+    cudaError_t e = launch_result(cudaStreamSynchronize(st));
     if (e != cudaSuccess) return cuda_fail(e, "new values");
     p->anorm = anorm > 0 ? anorm : 1.0;
     return 0;
