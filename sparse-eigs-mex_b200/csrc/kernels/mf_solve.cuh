@@ -57,6 +57,8 @@ constexpr int kBlkStrip = 64;        // columns of a forward strip, NR >= 8
 constexpr int kBlkTall = 16;         // row blocks of a backward strip, NR >= 8
 constexpr int kBwdCols = 64;         // columns of a backward tile at most
 constexpr int kListInts = 384;       // gather entries staged per task
+constexpr int kLongList = 16;        // longer gather lists are summed by many threads (grids have
+                                     // lists of up to 6, geometric graphs of up to 10)
 
 enum { SK_FWD = 0, SK_BWD = 1 };
 
@@ -68,7 +70,7 @@ struct STask {                       // 128 bytes: all a tile needs
     int j0, jn;                      // columns [j0, j0 + jn)
     int strip, nstrip, slot0, pad3;  // strip of its chunk, strips, first partial slot
     int pl0, pln, rl0, rln;          // gather entries of the pivots j0.. and of the rows
-    int has_child, pad0;
+    int has_child, pad0;             // has_child: 2 where the supernode has long gather lists
     long long g;                     // panel offset of (i0, j0)
     long long rows;                  // row-list offset of the supernode
     long long u;                     // update-vector offset (row c's entry)
@@ -297,20 +299,55 @@ SPX_DEV void sum_strips2(double2 (&s)[NCH], const double *p0, int64_t step, int 
 
 // entries q0 <= q < q1 of the gather list, summed in order; two loads at a
 // time in flight (most rows get one or two)
-SPX_DEV double sum_vals(const SolveArgs &a, const double *u, const int *ci, int lo, bool staged,
-                        int q0, int q1) {
+SPX_DEV double sum_vals(const double *u, const int32_t *cidx, const int *ci, int lo, bool staged,
+                        int q0, int q1, int *err) {
     double s = 0.0;
     for (int q = q0; q < q1; q += 2) {
         const bool two = q + 1 < q1;
-        const double *p0 = u + (staged ? ci[q - lo] : a.cidx[q]);
-        const double *p1 = two ? u + (staged ? ci[q + 1 - lo] : a.cidx[q + 1]) : p0;
+        const double *p0 = u + (staged ? ci[q - lo] : cidx[q]);
+        const double *p1 = two ? u + (staged ? ci[q + 1 - lo] : cidx[q + 1]) : p0;
         const double v0 = ld_val(p0);
         double v1 = 0.0;
         if (two) v1 = ld_val(p1);
-        s += got(v0, p0, a.err);
-        if (two) s += got(v1, p1, a.err);
+        s += got(v0, p0, err);
+        if (two) s += got(v1, p1, err);
     }
     return s;
+}
+
+// The gather lists of a supernode that has long ones (a vertex with thousands
+// of children below it): one row's entries follow one another at an L2 latency
+// for two, so a row of more than kLongList is summed by its thread's warp,
+// four loads a lane in flight, in a fixed order.  n rows, one a thread, with
+// list offsets at ptr[0..n]; their sums are added to out[0..n).  Solves: star
+// of 5,000 vertices 1.33 -> 0.070 ms, of 50,000 13.1 -> 0.45, 20,000 vertices
+// at three of ten hubs each 3.3 -> 0.27.  (Inlined: as a function of its own
+// it makes the kernel spill.)
+SPX_DEV void add_long_lists(const double *u, const int32_t *cidx, const int *ptr, int n, double *out,
+                            int *err) {
+    const int t = threadIdx.x, lane = t & 31;
+    const int q0 = t < n ? ptr[t] : 0, q1 = t < n ? ptr[t + 1] : 0;
+    const bool mine = q1 - q0 > kLongList;
+    double s = mine ? 0.0 : sum_vals(u, cidx, nullptr, 0, false, q0, q1, err);
+    for (unsigned m = __ballot_sync(0xffffffffu, mine); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int p0 = __shfl_sync(0xffffffffu, q0, src), p1 = __shfl_sync(0xffffffffu, q1, src);
+        double v = 0.0;
+        for (int q = p0 + lane; q < p1; q += 32 * 4) {
+            int at[4];
+            double x[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) at[e] = q + 32 * e < p1 ? cidx[q + 32 * e] : -1;
+#pragma unroll
+            for (int e = 0; e < 4; e++) x[e] = at[e] >= 0 ? ld_val(u + at[e]) : 0.0;
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (at[e] >= 0) v += got(x[e], u + at[e], err);
+        }
+        v = warp_sum(v);
+        if (lane == src) s = v;
+    }
+    if (t < n) out[t] += s;
 }
 
 // ---- one right-hand side ------------------------------------------------
@@ -346,11 +383,19 @@ SPX_DEV void vec_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
     double bsum = 0.0;
     if (k.probe_at) got(pv, pp, a.err);
     nx.take(a);
-    if (k.has_child) {
-        if (t < jn) bv += sum_vals(a, w.cur, l.ci, k.pl0, staged, l.cp[t], l.cp[t + 1]);
-        if (below) bsum = sum_vals(a, w.cur, l.ri, k.rl0, staged, l.rp[t], l.rp[t + 1]);
+    if (k.has_child == 2) {
+        // into the vector segment: the columns' sums with b, the rows' behind it
+        double *rows = sh.vec + kVecStrip;
+        const int r0 = k.strip == k.nstrip - 1 ? min(k.nrow, max(0, k.c - k.i0)) : k.nrow;
+        sh.vec[t] = bv;
+        if (r0 + t < k.nrow) rows[r0 + t] = 0.0;
+        add_long_lists(w.cur, a.cidx, l.cp, jn, sh.vec, a.err);
+        add_long_lists(w.cur, a.cidx, l.rp + r0, k.nrow - r0, rows + r0, a.err);
+    } else if (k.has_child) {
+        if (t < jn) bv += sum_vals(w.cur, a.cidx, l.ci, k.pl0, staged, l.cp[t], l.cp[t + 1], a.err);
+        if (below) bsum = sum_vals(w.cur, a.cidx, l.ri, k.rl0, staged, l.rp[t], l.rp[t + 1], a.err);
     }
-    if (t < jn) sh.vec[t] = bv;
+    if (t < jn && k.has_child != 2) sh.vec[t] = bv;
     nx.read(a);
     mbar_wait(&sh.pfull, ph, a.err);
     __syncthreads();
@@ -379,7 +424,7 @@ SPX_DEV void vec_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
             own += sum_strips(p0, kVecRows, k.nstrip - 1, a.err);
             const int ii = k.i0 + t;
             if (ii < k.c) put(w, a.o_yf + k.first + ii, own);
-            else put(w, k.u + (ii - k.c), bsum - own);
+            else put(w, k.u + (ii - k.c), (k.has_child == 2 ? sh.vec[kVecStrip + t] : bsum) - own);
         }
     }
     nx.stage(a, next, sh);          // this task's tile and lists are done with
@@ -462,6 +507,60 @@ SPX_DEV double2 brhs2(const SolveArgs &a, int64_t row, int col) {
                         col + 1 < a.nr ? __ldg(a.bc + (int64_t)(col + 1) * a.ldb + row) : 0.0);
 }
 
+// The lists of more than kLongList entries among a forward tile's columns (cp,
+// jn of them) and rows r0 <= r < nrow (rp), by the whole block: a thread takes
+// a pair of right-hand sides and every so-and-so-many'th entry, four loads in
+// flight; the shares are added in order.  Columns' sums are added to the
+// vector segment at vec, rows' are left in the second half of it (see
+// blk_long_rows).  A star of 5,000 vertices, 24 right-hand sides: 1.72 -> 0.14
+// ms a solve.
+template <int NR>
+SPX_DEV double *blk_long_rows(double *vec) {
+    return vec + kBlkStrip * SShared<NR>::SEG + kBlkThreads / (NR / 2) * NR;
+}
+template <int NR>
+SPX_DEV void blk_long_lists(const double *u, const int32_t *cidx, const int *cp, int jn,
+                            const int *rp, int r0, int nrow, double *vec, int *err) {
+    constexpr int H = NR / 2, NS = kBlkThreads / H, SEG = SShared<NR>::SEG;
+    static_assert(kBlkStrip * SEG + NS * NR + kBlkRows * NR <= kBlkTall * 16 * SEG, "long lists");
+    double *part = vec + kBlkStrip * SEG, *rows = blk_long_rows<NR>(vec);
+    const int t = threadIdx.x, h = t % H, sl = t / H;
+    __syncthreads();                                      // the segment is written
+    for (int e = 0; e < jn + nrow - r0; e++) {
+        const bool pivot = e < jn;
+        const int *p = pivot ? cp + e : rp + r0 + (e - jn);
+        const int q0 = p[0], q1 = p[1];
+        if (q1 - q0 <= kLongList) continue;               // for every thread
+        double2 s = make_double2(0.0, 0.0);
+        for (int q = q0 + sl; q < q1 && sl < NS; q += 4 * NS) {
+            const double *src[4];
+            double2 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                src[i] = u + (int64_t)(q + NS * i < q1 ? cidx[q + NS * i] : 0) * NR + 2 * h;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                x[i] = q + NS * i < q1 ? ld_val2(src[i]) : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (q + NS * i < q1) {
+                    const double2 v = got2(x[i], src[i], err);
+                    s.x += v.x;
+                    s.y += v.y;
+                }
+        }
+        if (sl < NS) *reinterpret_cast<double2 *>(part + sl * NR + 2 * h) = s;
+        __syncthreads();
+        if (t < NR) {
+            double v = 0.0;
+            for (int i = 0; i < NS; i++) v += part[i * NR + t];
+            if (pivot) vec[e * SEG + t] += v;
+            else rows[(r0 + e - jn) * NR + t] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // rows x columns (64 x jn) times (jn x NR): warp w holds rows 8 w .. 8 w + 7
 template <int NR>
 SPX_DEV void blk_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &next, SNext<NR> &nx,
@@ -496,6 +595,7 @@ SPX_DEV void blk_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
             const int e = t + kBlkThreads * p, jj = e / H, h = e % H;
             q0[p] = jj < jn ? l.cp[jj] : 0;
             q1[p] = jj < jn ? l.cp[jj + 1] : 0;
+            if (k.has_child == 2 && q1[p] - q0[p] > kLongList) q1[p] = q0[p];
             s0[p] = w.cur + (int64_t)(q0[p] < q1[p] ? entry(q0[p]) : 0) * NR + 2 * h;
             s1[p] = w.cur + (int64_t)(q0[p] + 1 < q1[p] ? entry(q0[p] + 1) : 0) * NR + 2 * h;
             z0[p] = z1[p] = make_double2(0.0, 0.0);
@@ -527,9 +627,21 @@ SPX_DEV void blk_fwd(const SolveArgs &a, const SVals &w, const STask &k, STask &
     double2 add[NCH];
 #pragma unroll
     for (int ch = 0; ch < NCH; ch++) add[ch] = make_double2(0.0, 0.0);
+    if (k.has_child == 2) {
+        // rows below the pivots, of the chunk's finishing strip
+        const int r0 = min(k.nrow, max(0, k.c - k.i0));
+        blk_long_lists<NR>(w.cur, a.cidx, l.cp, jn, l.rp, r0, finish ? k.nrow : r0, sh.vec, a.err);
+    }
     if (k.has_child && finish && lr < k.nrow && ii >= k.c) {
-        const int q1 = l.rp[lr + 1];
-        for (int q = l.rp[lr]; q < q1; q++) {
+        const int q0 = l.rp[lr], n = l.rp[lr + 1] - q0;
+        const bool summed = k.has_child == 2 && n > kLongList;
+        if (summed)
+#pragma unroll
+            for (int ch = 0; ch < NCH; ch++)
+                add[ch] = *reinterpret_cast<const double2 *>(blk_long_rows<NR>(sh.vec) + lr * NR +
+                                                             8 * ch + 2 * tq);
+        const int q1 = summed ? q0 : q0 + n;
+        for (int q = q0; q < q1; q++) {
             const double *src = w.cur + (int64_t)(staged ? l.ri[q - k.rl0] : a.cidx[q]) * NR + 2 * tq;
             double2 z[NCH];
 #pragma unroll

@@ -257,7 +257,7 @@ static void plan_factor_tasks(const spx_symbolic &S, const int64_t *gptr,
 // them: its first task and its first partial-sum slot.
 struct SPlanNode {
     int first, c, r, parent;
-    int has_child, probe;            // probe: see STask, of a forward task
+    int has_child, probe;            // see STask; probe: of a forward task
     long long g, rows, u;
 };
 struct SPlanEntry { int s, task0, slot0; };
@@ -450,12 +450,12 @@ static int solve_config(int *grid) {
         cudaGetLastError();
         return SPEIGS_ERR_INTERNAL;
     }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf_solve<NR>, SShared<NR>::kThreads, sizeof(SShared<NR>));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf_solve<NR>, SShared<NR>::kThreads,
+                                                  sizeof(SShared<NR>));
     if (per_sm <= 0 || nsm <= 0) return SPEIGS_ERR_INTERNAL;
     *grid = nsm * per_sm;
     return 0;
 }
-
 template <class Tp>
 static int dmalloc(Tp **p, size_t cnt, cudaStream_t st) {
     int dev = 0;
@@ -537,6 +537,7 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
         std::vector<int32_t> atpos, acolj, asrc;
         std::atomic<int> dup{0};
         std::vector<int32_t> cptr(nrows_total_ + 1, 0), cidx;
+        std::vector<char> longlist(ns, 0);          // some gather list is long
         std::vector<int32_t> cbnd;
         std::vector<FNodeH> fnode(ns);
         std::vector<FChildH> fchild(S.child_ptr[ns]);
@@ -596,7 +597,7 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
                     const int ch = S.child_list[q];
                     const int cc = S.sfirst[ch + 1] - S.sfirst[ch];
                     for (int64_t t = S.rowptr[ch] + cc; t < S.rowptr[ch + 1]; t++)
-                        cptr[S.rowptr[par] + S.relmap[t] + 1]++;
+                        if (++cptr[S.rowptr[par] + S.relmap[t] + 1] > kLongList) longlist[par] = 1;
                 }
             for (int64_t g = 0; g < nrows_total_; g++) cptr[g + 1] += cptr[g];
             cidx.assign(cptr[nrows_total_], 0);
@@ -640,6 +641,8 @@ template <> int MultifrontalPlanT<Real>::init(const spx_symbolic &S, const int64
             m.u = uptr[s];
         }
         side.wait();
+        for (int32_t s = 0; s < ns; s++)
+            if (longlist[s]) pnode[s].has_child = 2;
         int rc = 0;
         rc = rc ? rc : dupload(&d_cbnd_, cbnd.data(), cbnd.size(), st);
         rc = rc ? rc : dupload((FNodeH **)&d_fnode_, fnode.data(), fnode.size(), st);
