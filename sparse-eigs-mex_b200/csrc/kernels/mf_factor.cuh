@@ -192,6 +192,55 @@ SPX_DEV void acc_each(const Acc &acc, int m0, int n0, Fn f) {
             for (int i = 0; i < 4; i++) f(m0 + 8 * i + g, n0 + 8 * j + 2 * t + e, acc[i][j][e]);
 }
 
+// Up to 32 children, one a lane (update matrix U of order nb, its rows' places
+// rm), that touch the tile with at most kTiny rows (update rows ia .. ia + hi)
+// and kTiny columns (ja .. ja + wj) each: every lane loads its child's
+// entries, and for one place (u, v) of them after the other the lanes that meet
+// in an entry of the tile sum theirs, in the children's order, and add the sum.
+// A vertex with many small children below it is bound by their loads' latency:
+// one child at a time takes 0.7 us each, this 0.14.  Star of 5,000 vertices
+// 3.65 -> 0.74 ms, 20,000 vertices at three of ten hubs each 27.3 -> 9.1, grids
+// the same (their fronts have up to 25 children).
+constexpr int kTiny = 4;
+__device__ __noinline__ void add_tiny_children(const Real *U, const int32_t *rm, double *S, int nb, int ia,
+                                               int hi, int ja, int wj, int ra, int ca) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int ri[kTiny], rj[kTiny];
+    double x[kTiny][kTiny];
+#pragma unroll
+    for (int u = 0; u < kTiny; u++) {
+        ri[u] = u < hi && wj > 0 ? rm[ia + u] - ra : -1;
+        rj[u] = u < wj && hi > 0 ? rm[ja + u] - ca : -1;
+        if ((rj[u] & 3) != wid) rj[u] = -1;              // another warp's column
+    }
+#pragma unroll
+    for (int v = 0; v < kTiny; v++)
+#pragma unroll
+        for (int u = 0; u < kTiny; u++) {
+            const int i = ia + u, j = ja + v;
+            x[u][v] = 0.0;
+            if (ri[u] >= 0 && rj[v] >= 0 && i >= j)
+                x[u][v] = (double)__ldcg(U + utile(nb, i / FT, j / FT) + tix<Real>(i % FT, j % FT));
+        }
+#pragma unroll
+    for (int v = 0; v < kTiny; v++)
+#pragma unroll
+        for (int u = 0; u < kTiny; u++) {
+            const bool mine = ri[u] >= 0 && rj[v] >= 0 && ia + u >= ja + v;
+            if (!__any_sync(full, mine)) continue;
+            const int at = mine ? tix<double>(ri[u], rj[v]) : -1 - lane;
+            const unsigned same = __match_any_sync(full, at);
+            double s = 0.0;
+            for (unsigned m = same; __any_sync(full, m != 0); m &= m - 1) {
+                const double y = __shfl_sync(full, x[u][v], m ? __ffs(m) - 1 : lane);
+                if (m) s += y;
+            }
+            if (mine && lane == __ffs(same) - 1) S[at] += s;
+            __syncwarp();
+        }
+}
+
 // S(i, j) = the assembled tile of rows [ra, ra + h) x columns [ca, ca + w)
 // of the front: children's update matrices in child order, then A and the
 // shift.  Each warp owns the target columns j with j % 4 = its index, so the
@@ -217,6 +266,10 @@ SPX_DEV void assemble(const FactorArgs &a, const FNode &nd, double *S, int I, in
             wj = bd[J + 1] - ja;
         }
         unsigned live = __ballot_sync(full, hi > 0 && wj > 0);
+        if (__popc(live) >= 4 && __all_sync(full, hi <= kTiny && wj <= kTiny)) {
+            add_tiny_children(a.F + ch.uptr, a.relmap + ch.relmap, S, ch.nb, ia, hi, ja, wj, ra, ca);
+            continue;
+        }
         while (live) {
             const int src = __ffs(live) - 1;
             live &= live - 1;
