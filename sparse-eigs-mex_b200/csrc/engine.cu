@@ -1453,7 +1453,7 @@ int plan_from_csr(HostCSR &A, speigs_which which, const speigs_opts &o, double a
     p->anorm = anorm;
     p->mf.mixed = (which == SPEIGS_SM && ext && ext->precision == SPEIGS_B200_MIXED);
     if (ext && ext->refine_max > 0) p->refine.max_steps = ext->refine_max;
-    if (ext && ext->refine_tol > 0) p->refine_tol_user = ext->refine_tol;
+    if (ext && ext->refine_tol > 0) p->refine.tol = p->refine_tol_user = ext->refine_tol;
     if (p->stream.err != cudaSuccess) { int rc = cuda_fail(p->stream.err, "stream"); speigs_plan_destroy(p); return rc; }
     cudaStream_t st = p->stream.s;
     const int n = p->A.n;
