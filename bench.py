@@ -326,13 +326,11 @@ def run_metric(args, pkg, wl, ctx):
             raise RuntimeError(f"mpnn forward rc={rc}")
         Y_t.copy_(Y32.t())
         torch.cuda.synchronize()
-        cache = os.path.join(ROOT, "gpurun_out", "tune_cache.json") \
-            if os.path.isdir(os.path.join(ROOT, "gpurun_out")) else None
         t_tune = time.perf_counter()
         for pname, prec in (("fp64", s.FP64), ("mixed", s.MIXED)):
             e = pkg.tune.tune_operator(A_t, k, s.SM, prec, warm_ptr=Y_t.data_ptr(), warm_cols=P,
                                        tol=TOL, blocks=(-1, 8, 16, 24), ncvs=(64, 96, 128),
-                                       reps=1, cache=cache, lib=lib)
+                                       reps=1, lib=lib)
             tuning[pname] = e["best"]
             tuning[pname + "_candidates"] = [
                 {kk: r.get(kk) for kk in ("block", "ncv", "ms", "ok", "block_solves")}

@@ -386,8 +386,10 @@ __global__ void __launch_bounds__(kGsThreads, 2) ts_kernel(TsParams p, int per) 
 // Update and dot products in one read of V, for up to M columns: a thread holds
 // its row of V in registers between the two and the columns' sums over its
 // rows, which are added over the block once at the end.  100^3 rows, 14 columns
-// on average: 30.3 us when the products read V again out of L2, 24 now (the
-// whole iteration 11.05 -> 10.2 ms); at 64^3 rows, V in L2, the two are equal.
+// on average: 30.3 us when the products read V again out of L2, 24 now (a
+// solve of 47 steps and 3 restarts 11.05 -> 10.1 ms); at 64^3 rows, V in L2, the
+// two are equal.  M: powers of two, the default basis size (20), and the widest
+// whose sums fit the registers; 20 and 40 spill a few (36 bytes) all the same.
 constexpr int kUdThreads = 256;
 // blocks an SM that the registers allow
 __host__ __device__ constexpr int ud_blocks(int M) { return M <= 8 ? 3 : M <= 20 ? 2 : 1; }

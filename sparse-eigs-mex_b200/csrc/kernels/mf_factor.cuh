@@ -6,8 +6,8 @@
 // (left-looking): it assembles the tile (entries of A, the shift, the
 // children's update matrices), subtracts the products of the finished tiles
 // to its left and finishes it.  Tasks come from an atomic queue sorted by
-// the length of the path that still hangs on them, and wait on a flag per
-// tile, so there is no barrier between column blocks or tree levels and no
+// the earliest time they can run (the longest path below them), and wait on a
+// flag per tile, so there is no barrier between column blocks or tree levels and no
 // launch per step.  The queue order is topological (a task waits only for
 // tasks before it, which running blocks hold), so the waits cannot deadlock
 // whatever number of blocks is resident; they are bounded all the same.

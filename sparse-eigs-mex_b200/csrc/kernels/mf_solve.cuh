@@ -93,8 +93,8 @@ struct SolveArgs {
     int *sync;                       // queue, blocks gone, copy in use
     int *err;
     const double *bc;                // right-hand sides, column-major, original order
-    double *xc;                      // results; every write follows the whole forward
-                                     // pass, so xc may be bc
+    double *xc;                      // results; a tree's writes follow its whole forward
+                                     // pass, so xc may be bc (other overlaps may not)
     int64_t ldb, ldx;
     int nr;                          // columns given (the rest read as zero)
     int accumulate;                  // xc += the solution (else xc = it)

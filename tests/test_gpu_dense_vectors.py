@@ -1,7 +1,7 @@
-"""The few-pairs solver's back-transform (one warp a column up to n = 512, in 8 or 16 registers a
-lane, a block a column above), its bisection (512 points a round) and its quotients (256 rows at
-a time, four threads a row) at the orders where a lane, a register or a chunk of rows or columns
-begins.
+"""The few-pairs solver's back-transform (a block of 128 threads a column, with 2, 8 or 32 entries a
+thread up to n = 256, 1,024 and above), its bisection (512 points a round) and its quotients (256
+rows at a time, four threads a row) at the orders where a warp, an entry or a chunk of rows or
+columns begins.
 
 Tolerances: backward error n eps |A| for the reduction and the back-transform together, with a
 factor of ten; the quotients are in twice the precision, so an eigenvalue is off by the square

@@ -1,4 +1,4 @@
-"""Mixed precision (FP32 factor on the TF32 tensor cores + FP64 refinement of
+"""Mixed precision (FP32 factor, FP64 products of its tiles + FP64 refinement of
 every solve) against the plain FP64 path and the CPU reference.
 
 The refined operator must agree with an FP64 solve to the refinement target,
@@ -84,9 +84,8 @@ def test_mixed_singular_takes_shift(lib, pkg):
 def test_fp32_factor_is_fp32_accurate(lib, pkg, case):
     """One solve with the FP32 factor alone (refine_tol = 1 accepts it
     without a correction): its backward error is at the FP32 level.  The
-    trailing updates take three TF32 products (hi.hi + hi.lo + lo.hi) on the
-    tensor cores; with the head alone the factor would carry TF32 errors
-    (~1e-3), far above this bound."""
+    factor's products are FP64 products of FP32 tiles; of TF32 ones it would
+    carry errors of ~1e-3, far above this bound."""
     torch = pytest.importorskip("torch")
     import scipy.sparse as sp
     w = pkg.workloads
